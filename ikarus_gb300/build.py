@@ -23,7 +23,7 @@ NVCC_FLAGS = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-
                      "-Xptxas", "-warn-spills"]
 CXX_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-Wall", "-Wno-unused-function", "-I" + os.path.join(CUDA_HOME, "include")]
 
-CU_SOURCES = ["element.cu", "element_eas.cu", "element_eas_hyper.cu", "sparse.cu", "solver.cu", "spmv_staged.cu", "cg_persistent.cu", "cg_coarse.cu", "noalloc.cu", "mlp.cu", "batched.cu", "coarse.cu", "krylov.cu"]
+CU_SOURCES = ["element.cu", "element_eas.cu", "element_eas_hyper.cu", "sparse.cu", "solver.cu", "spmv_staged.cu", "cg_persistent.cu", "cg_halo.cu", "cg_coarse.cu", "noalloc.cu", "mlp.cu", "batched.cu", "coarse.cu", "krylov.cu"]
 CPP_SOURCES = ["host.cpp", "batched_host.cpp", "predictor.cpp", "path_following.cpp", "krylov.cpp", "operators.cpp",
                "newton_graph.cpp"]
 

@@ -326,6 +326,7 @@ struct ikr_asm_s {
   bool idbc_vals_valid = false;
   // pattern
   int64_t nb = 0, npad = 0;
+  uint64_t pattern_id = 0;  // of every pattern built in this process, from 1
   int nslices = 0;
   DBuf<int32_t> ne_ptr, ne_elems;  // elements of every node, ascending (row-tangent kernel)
   // FP32 tangent kernel: 0 = not chosen yet, 1 = coloured element kernel, 2 = row kernel, 3 = element blocks +
@@ -450,6 +451,8 @@ struct ikr_asm_s {
     f->check_status();
     if (fp32) val32.alloc(9 * npad);
     else val64.alloc(9 * npad);
+    static std::atomic<uint64_t> patterns{0};
+    pattern_id = ++patterns;
   }
   // block id of CSR entry k (the (k - row_ptr[r])-th block of row r)
   int64_t block_id(int r, int64_t k) const { return (slice_off_h[r >> 5] + (k - row_ptr_h[r])) * 32LL + (r & 31); }
@@ -473,8 +476,16 @@ struct ikr_ls_s {
   ikr::PcgWork w;
   DBuf<double> dx, dp, dq, dmv, pa, pb, scal;
   DBuf<float> fx, fp, fq, fmv;
-  DBuf<double> dz, dr, dp1, dzb, dw0, dw1, pc;  // dzb / fzb, dw / fw: one-reduction CG (second z, w = M^-1 q)
-  DBuf<float> fz, fr, fp1, fzb, fw0, fw1;
+  DBuf<double> dz, dr, dp1, pc;
+  DBuf<float> fz, fr, fp1;
+  // split of the system for the one-reduction CG (cg_halo.cu), made once per pattern
+  struct HaloSet {
+    uint64_t pattern = 0;  // the assembler pattern it belongs to (0: none yet)
+    uint64_t made = 0;     // plans made by this solver
+    ikr::HaloPlan P;
+    DBuf<int32_t> slice0, cnt, halo;
+    DBuf<uint16_t> col16;
+  } ho;
   double* scal_h = nullptr;
   cudaEvent_t ev[2] = {nullptr, nullptr};
   cudaEvent_t tev[2] = {nullptr, nullptr};  // timing events of the SpMV tuner
@@ -578,17 +589,14 @@ struct ikr_ls_s {
     tuned_for = nullptr;
     if (fp32) {
       fx.alloc(n), fr.alloc(n), fz.alloc(n), fp.alloc(n), fp1.alloc(n), fq.alloc(n), fmv.alloc(9 * (size_t)nr);
-      fzb.alloc(n), fw0.alloc(n), fw1.alloc(n);
       w.x = fx.p, w.r = fr.p, w.z = fz.p, w.p0 = fp.p, w.p1 = fp1.p, w.q = fq.p, w.minv = fmv.p;
-      w.z2 = fzb.p, w.w0 = fw0.p, w.w1 = fw1.p;
     } else {
       dx.alloc(n), dr.alloc(n), dz.alloc(n), dp.alloc(n), dp1.alloc(n), dq.alloc(n), dmv.alloc(9 * (size_t)nr);
-      dzb.alloc(n), dw0.alloc(n), dw1.alloc(n);
       w.x = dx.p, w.r = dr.p, w.z = dz.p, w.p0 = dp.p, w.p1 = dp1.p, w.q = dq.p, w.minv = dmv.p;
-      w.z2 = dzb.p, w.w0 = dw0.p, w.w1 = dw1.p;
     }
-    pc.alloc(16 * (size_t)w.grid);
+    pc.alloc(ikr::kHaloWords);
     w.part_c = pc.p;
+    ho.pattern = 0;
     pa.alloc(2 * (size_t)w.grid);  // two-kernel CG: 1 per block; persistent CG: 2 per CTA (parity)
     pb.alloc(4 * (size_t)w.grid);  // two-kernel CG: 2 per block; persistent CG: 4 per CTA
     scal.alloc(ikr::kNScal);
@@ -659,6 +667,45 @@ struct ikr_ls_s {
     }
   }
 
+  // The halo plan of the assembler's pattern; w.halo stays null where the split does not fit a 16-bit local index or
+  // the kernel's shared memory (pcg_halo_eligible checks the latter per variant).
+  void halo_plan(ikr_asm a) {
+    if (ho.pattern == a->pattern_id) return;
+    if (ho.pattern) tuned_for = nullptr;  // another pattern of the same assembler object: its kernel choice as well
+    ho.pattern = a->pattern_id;
+    ++ho.made;
+    w.halo = nullptr;
+    const int nn = a->fes->nn;
+    if (nn > ikr::halo_max_rows()) return;
+    cudaStream_t s = a->fes->stream;
+    ikr::HaloPlan& P = ho.P;
+    P = ikr::HaloPlan{};
+    P.chunk = ikr::halo_chunk(nn, w.sms);
+    P.n_cta = ikr::halo_ctas(nn, w.sms);
+    P.halo_cap = std::min(nn, 12 * 1024);
+    ho.slice0.alloc(P.n_cta + 1);
+    ho.cnt.alloc(P.n_cta);
+    ho.halo.alloc((size_t)P.n_cta * P.halo_cap);
+    ho.col16.alloc(a->npad);
+    P.slice0 = ho.slice0.p, P.halo_cnt = ho.cnt.p, P.halo = ho.halo.p, P.col16 = ho.col16.p;
+    CK(ikr::launch_halo_plan(a->bsr(), P, ho.slice0.p, ho.cnt.p, ho.halo.p, ho.col16.p, s));
+    count(1);
+    std::vector<int32_t> cnt(P.n_cta);
+    ho.cnt.download(cnt.data(), cnt.size(), s);
+    CK(cudaStreamSynchronize(s));
+    P.max_halo = *std::max_element(cnt.begin(), cnt.end());
+    if (P.max_halo > P.halo_cap) return;
+    for (int c = 0; c < P.n_cta; ++c) {
+      const int64_t S = a->nslices;
+      const int sa = P.chunk == 32 ? (int)(c * S / P.n_cta) : c * P.chunk / 32;
+      const int sb = P.chunk == 32 ? (int)((c + 1) * S / P.n_cta) : sa + 1;
+      const int cols = a->slice_off_h[sb] - a->slice_off_h[sa];
+      P.max_ns = std::max(P.max_ns, sb - sa);
+      P.max_units = std::max(P.max_units, P.chunk == 32 ? cols : (cols * P.chunk + 31) / 32);
+    }
+    w.halo = &P;
+  }
+
   void factorize(ikr_asm a) {
     if (tag == IKR_SOLVER_NONE) fail(IKR_ERR_INVALID_STATE, "SolverTypeTag::none has no linear solver");
     if (dense) fail(IKR_ERR_NOT_IMPLEMENTED, "This solver does not support solving with sparse matrices.");
@@ -670,6 +717,7 @@ struct ikr_ls_s {
     factorized = true;
     w.coarse = 0;
     if (coarse_req > 0) coarse_operator(a);  // before the tuner: the fused kinds are timed with it
+    else if (tag != IKR_SOLVER_GPU_PCG_BATCHED) halo_plan(a);
     if (tag != IKR_SOLVER_GPU_PCG_BATCHED && tuned_for != a) tune(a);
     if (coarse_req > 0) {
       if (persistent())
@@ -978,11 +1026,21 @@ struct ikr_ls_s {
     if (spmv_req < 0) {
       // the kinds are compared with a mid L2 keep share (the share changes their ranking), kind 0 has none
       constexpr double kProbeKeep = 0.45;
-      for (int k = 0; k <= ikr::spmv_staged_variants(); ++k) {
+      // The one-reduction kernel wherever a split fits: it was the fastest persistent form at every size timed (table
+      // in cg_halo.cu), so only its variants are compared
+      bool halo = false;
+      for (int v = 0; v < ikr::kHaloVariants && coarse_req == 0; ++v) {
+        if (!ikr::pcg_halo_eligible(w, v)) continue;
+        halo = true;
+        const int kind = first_coarse_kind() - ikr::kHaloVariants + v;
+        const double us = time_persistent(kind, kProbeKeep);
+        if (us < best) best = us, best_kind = kind;
+      }
+      for (int k = 0; k <= ikr::spmv_staged_variants() && !halo; ++k) {
         const double us = time_it(k, k > 0 ? kProbeKeep : 0.0);
         if (us < best) best = us, best_kind = k;
       }
-      for (int v = 0; v < ikr::pcg_persistent_variants() && coarse_req == 0; ++v) {
+      for (int v = 0; v < ikr::pcg_persistent_variants() - ikr::kHaloVariants && coarse_req == 0 && !halo; ++v) {
         if (!ikr::pcg_persistent_eligible(A, w, v)) continue;
         const double us = time_persistent(first_persistent_kind() + v, kProbeKeep);
         if (us < best) best = us, best_kind = first_persistent_kind() + v;
@@ -1012,7 +1070,9 @@ struct ikr_ls_s {
       fail(IKR_ERR_ARG, "the persistent CG variant does not fit this system (too many slices per warp)");
     }
     double best_keep = keep_req >= 0.0 ? keep_req : 0.0;
-    if (keep_req < 0.0 && best_kind > 0) {
+    const int hv = best_kind - (first_coarse_kind() - ikr::kHaloVariants);
+    const bool in_smem = hv >= 0 && hv < ikr::kHaloVariants && ikr::pcg_halo_eligible(w, hv) && !ikr::pcg_halo_streams(w, hv);
+    if (keep_req < 0.0 && best_kind > 0 && !in_smem) {
       best = time_kind(best_kind, 0.0);
       for (double f : {0.3, 0.45, 0.6, 0.75}) {
         const double us = time_kind(best_kind, f);

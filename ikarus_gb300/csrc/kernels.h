@@ -204,6 +204,21 @@ enum PcgScal : int {
   kTicket = 12, // slots 12-14 hold six 32-bit tickets of the last-block reductions (the fifth: coarse.cu)
   kNScal = 16
 };
+// cg_halo.cu -- split of a system's rows over n_cta CTAs and, per CTA, the rows outside its own that its blocks refer
+// to.  chunk 32: whole slices [slice0[c], slice0[c + 1]); 4, 8, 16: rows [c chunk, (c + 1) chunk).  col16 holds, per
+// padded block, the column's index among the CTA's own rows, then its halo rows.
+struct HaloPlan {
+  int n_cta = 0, chunk = 32;
+  int halo_cap = 0;                   // entries of halo per CTA
+  int max_halo = 0, max_ns = 0, max_units = 0;  // largest halo, slices and block columns (chunk units) of a CTA
+  const int32_t* slice0 = nullptr;    // n_cta + 1
+  const int32_t* halo_cnt = nullptr;  // n_cta
+  const int32_t* halo = nullptr;      // n_cta x halo_cap, ascending
+  const uint16_t* col16 = nullptr;    // n_padded
+};
+constexpr int kHaloVariants = 2;      // warps per CTA: 16 and 8 in FP32, 8 and 16 in FP64
+constexpr int kHaloWords = 2 * 5 * 8 * 160 * 2;  // doubles of part_c: 2 parities x 5 sums x 8 copies x 160 CTAs x 16 B
+
 struct PcgWork {
   int n_rows = 0;     // block rows
   bool fp32 = false;
@@ -222,11 +237,9 @@ struct PcgWork {
   int spmv_kind = 0;           // 0: direct loads (solver.cu); 1 + v: staged variant v (spmv_staged.cu);
                                // 1 + staged variants + v: persistent CG variant v (cg_persistent.cu)
   int64_t keep_g = 0;          // staged: matrix blocks [0, keep_g) are copied with an L2 evict_last policy
-  // one-reduction persistent CG (variants 4 and 5 of cg_persistent.cu): a second z buffer, the two buffers of
-  // w = M^-1 q and 16 partials per grid CTA
-  void* z2 = nullptr;
-  void* w0 = nullptr;
-  void* w1 = nullptr;
+  // one-reduction persistent CG (cg_halo.cu): the system's split (nullptr: none fits) and the tagged words of its
+  // sums, zeroed by the init kernel
+  const HaloPlan* halo = nullptr;
   double* part_c = nullptr;
   // 1: a coarse correction (coarse.cu) follows the init and update kernels, which then leave r.D^-1 r in kRzF
   // and let it set r.z and beta
@@ -283,6 +296,15 @@ void launch_coarse_probe(const Coarse& C, int colour, double* V, cudaStream_t s)
 void launch_coarse_galerkin(const Coarse& C, const double* W, double* part, cudaStream_t s);
 int pcg_persistent_variants();
 bool pcg_persistent_eligible(const Bsr& A, PcgWork& w, int variant);
+// cg_halo.cu -- the last kHaloVariants persistent variants where the system has a split that fits
+int halo_chunk(int n_rows, int sms);
+int halo_ctas(int n_rows, int sms);
+int halo_max_rows();
+cudaError_t launch_halo_plan(const Bsr& A, const HaloPlan& P, int32_t* slice0, int32_t* cnt, int32_t* halo,
+                             uint16_t* col16, cudaStream_t s);
+bool pcg_halo_eligible(const PcgWork& w, int variant);
+bool pcg_halo_streams(const PcgWork& w, int variant);
+cudaError_t launch_pcg_halo(const Bsr& A, PcgWork& w, int variant, cudaStream_t s);
 cudaError_t launch_pcg_persistent(const Bsr& A, PcgWork& w, int variant, cudaStream_t s);
 // the same solve for two right-hand sides with one matrix stream per iteration (w1 shares w0's matrix,
 // preconditioner, grid and L2 policy); part_a / part_b hold 4 and 8 doubles per grid CTA

@@ -127,9 +127,11 @@ __global__ void __launch_bounds__(kThreads) pcg_init_kernel(int n_rows, const T*
                                                             const double* __restrict__ b, T* x, T* r, T* z, T* pold,
                                                             double* part, double* scal, double rtol,
                                                             const double* __restrict__ rtol_dev, int max_iter,
-                                                            int coarse) {
+                                                            int coarse, double* words) {
   __shared__ double sh[32];
   __shared__ bool last;
+  if (words)  // the tagged words of the one-reduction CG's sums
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < kHaloWords; i += gridDim.x * blockDim.x) words[i] = 0.0;
   double rz = 0.0, rr = 0.0;
   for (int row = blockIdx.x * blockDim.x + threadIdx.x; row < n_rows; row += gridDim.x * blockDim.x) {
     const T rv[3] = {T(b[3 * row]), T(b[3 * row + 1]), T(b[3 * row + 2])};
@@ -254,11 +256,12 @@ void launch_pcg_init(const Bsr& A, PcgWork& w, const double* b, double rtol, int
   if (w.fp32)
     pcg_init_kernel<float><<<w.grid, kThreads, 0, s>>>(w.n_rows, (const float*)w.minv, b, (float*)w.x, (float*)w.r,
                                                         (float*)w.z, (float*)w.p1, w.part_b, w.scal, rtol, w.rtol_dev,
-                                                        max_iter, w.coarse);
+                                                        max_iter, w.coarse, w.halo ? w.part_c : nullptr);
   else
     pcg_init_kernel<double><<<w.grid, kThreads, 0, s>>>(w.n_rows, (const double*)w.minv, b, (double*)w.x,
                                                          (double*)w.r, (double*)w.z, (double*)w.p1, w.part_b, w.scal,
-                                                         rtol, w.rtol_dev, max_iter, w.coarse);
+                                                         rtol, w.rtol_dev, max_iter, w.coarse,
+                                                         w.halo ? w.part_c : nullptr);
 }
 
 void launch_pcg_spmv(const Bsr& A, PcgWork& w, int parity, cudaStream_t s) {
