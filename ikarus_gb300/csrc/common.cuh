@@ -22,6 +22,28 @@ __device__ __forceinline__ void ref_gradient_at_gp(int v, int q, T dxi[3]) {
   dxi[1] = ((v & 2) ? T(1) : T(-1)) * f0 * f2;
   dxi[2] = ((v & 4) ? T(1) : T(-1)) * f0 * f1;
 }
+// The same for one Gauss point and all nodes, without FP64 instructions: |dN_v/dxi_d| takes four values per direction,
+// by the node's bits in the other two directions (d = 0: bits 1, 2; 1: bits 0, 2; 2: bits 0, 1), its sign is bit d's.
+struct GpFactors {
+  double f[3][4];
+  __device__ __forceinline__ explicit GpFactors(int q) {
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const int a = (q >> (d == 0 ? 1 : 0)) & 1, b = (q >> (d == 2 ? 1 : 2)) & 1;
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        const int same = ((m & 1) == a) + ((m >> 1) == b);
+        f[d][m] = same == 2 ? kGaussHi * kGaussHi : same == 1 ? kGaussHi * kGaussLo : kGaussLo * kGaussLo;
+      }
+    }
+  }
+  // dN_v/dxi_d (v and d compile-time)
+  __device__ __forceinline__ double operator()(int v, int d) const {
+    const int a = (v >> (d == 0 ? 1 : 0)) & 1, b = (v >> (d == 2 ? 1 : 2)) & 1;
+    const double x = f[d][a + 2 * b];
+    return (v >> d) & 1 ? x : -x;
+  }
+};
 // dN_v/dxi at the element centre (1/2,1/2,1/2)
 template <typename T>
 __device__ __forceinline__ void ref_gradient_at_center(int v, T dxi[3]) {

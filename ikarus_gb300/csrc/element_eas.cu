@@ -245,11 +245,10 @@ void launch_eas_stress_at(const ElemArgs& a, int e0, int count, const double* xi
 
 int eas_geo_stride(int kind) { return kind == 1 ? 36 : (kind == 3 ? 34 : 10); }
 
-void launch_eas_element(const ElemArgs& a, int mode, bool fp32, const int32_t* list, int n, int base,
-                        cudaStream_t s) {
+void launch_eas_element(const ElemArgs& a, int mode, const int32_t* list, int n, int base, cudaStream_t s) {
   if (n <= 0) return;
-  if (a.material == 3) launch_eas_element_hyper(a, mode, fp32, list, n, base, s);  // element_eas_hyper.cu
-  else launch_eas_family<false>(a, mode, fp32, list, n, base, s);
+  if (a.material == 3) launch_eas_element_hyper(a, mode, list, n, base, s);  // element_eas_hyper.cu
+  else launch_eas_family<false>(a, mode, list, n, base, s);
 }
 
 void launch_eas_geometry(const ElemArgs& a, double* geo_out, cudaStream_t s) {

@@ -5,15 +5,21 @@
 // the strain functions easfunctions/{greenlagrangestrain,displacementgradient,displacementgradienttransposed}.hh
 // and the ansatz spaces easvariants/{linearandglstrains,displacementgradient,helperfunctions}.hh.
 //
-// Same decomposition as the displacement kernel: 8 lanes per element, lane = node I.  Per Gauss point the
-// lanes share F, S and the Voigt tangent C (each lane computes a few of its 36 entries into shared memory),
-// and each lane computes the enhanced-strain columns E_alpha(:,k) and C E_alpha(:,k) for k = I, I+8, ...
-// After the Gauss loop the element's D (n_alpha x n_alpha) is LU-factorised once per element (lane 0,
-// partial pivoting, FP64); every lane solves for its own D^{-1} L_I, and the condensed quantities
+// One element per block of 64 threads: eight lanes (lane = node I) for each of the eight Gauss points, because the work
+// at a point is about 1 800 dependent FP64 instructions a lane, which GB300 starts one per 16 cycles and SM and finishes
+// one per 60: an element whose points follow one another keeps a small mesh waiting for eight times that, and one lane
+// factorising D keeps the other seven.  Measured against eight lanes per element and one launch per colour, residual and
+// tangent with assembly: 10 elements 660 -> 60 us and 1 030 -> 80 us, 8 192 elements 2.34 -> 1.01 ms and 3.86 -> 1.63 ms.
+// The lanes of a point share F, S and the Voigt tangent C (each lane computes a few of its 36 entries into shared
+// memory), and each lane computes the enhanced-strain columns E_alpha(:,k) and C E_alpha(:,k) for k = I, I+8, ...
+// The points' shares of f, K, L, D and R~ are summed in point order through shared memory.  D (n_alpha x n_alpha) is
+// LU-factorised with a lane per row (partial pivoting, FP64), the 24 columns of D^{-1} L and D^{-1} R~ are solved with
+// a lane each, and the condensed quantities
 //   f_I -= L_I^T D^{-1} R~,   K_IJ -= L_I^T D^{-1} L_J        (enhancedassumedstrains.hh:291-296, 336-345)
-// are formed with the same 5-blocks-per-lane ownership as the displacement kernel.
-// D^{-1} R~ and D^{-1} L are cached per element (FP64) when the residual is assembled, so the internal-state
+// are formed by all 64 threads; K as the 40 blocks (I, I + d mod 8), d = 0..4, d = 1..3 transposed as well.
+// D^{-1} R~ and D^{-1} L are cached per element (FP64) when the residual is formed, so the internal-state
 // update alpha -= D^{-1} (R~ + L dd) (enhancedassumedstrains.hh:225-248) costs one pass over the cache.
+// The kernel writes element vectors and matrices; assembly gathers them (element.cu), in element order.
 //
 // The enhancement modes are rank one.  H9: H_p = s_p a_r (x) a_c with p = 3r + c, s_p = (detJ0/detJ)(2 xi_c - 1)
 // and a_k the k-th column of J0^{-T} (easvariants/displacementgradient.hh:136-161, helperfunctions.hh:27-36).
@@ -39,21 +45,26 @@ __constant__ int kF2[21] = {-1, -1, -1, -1, -1, -1, -1, -1, -1, 1, 2, 1, 2, 2, 2
 
 template <int NA>
 struct EasCfg {
-  static constexpr int EPB = NA <= 9 ? 8 : 4;  // elements per 64/32-thread block
   static constexpr int NT = NA * (NA + 1) / 2; // packed upper triangle of D
   static constexpr int DSH = (NT + 7) / 8;     // D entries per lane
   static constexpr int RSH = (NA + 7) / 8;     // R~ entries per lane
-  // shared memory per element (doubles)
+  // shared memory of a Gauss point (doubles)
   static constexpr int O_DN = 0;               // 8 x 3   modified nodal gradients
   static constexpr int O_C6 = O_DN + 24;       // 36      Voigt tangent
   static constexpr int O_EA = O_C6 + 36;       // NA x 6  E_alpha columns
   static constexpr int O_CEA = O_EA + 6 * NA;  // NA x 6  C E_alpha columns
-  static constexpr int O_GEO = O_CEA + 6 * NA; // 36      T0^{-1} (GL)
-  static constexpr int O_D = O_GEO + 36;       // NA x NA
-  static constexpr int O_RT = O_D + NA * NA;   // NA
-  static constexpr int O_Y = O_RT + NA;        // 8 x NA x 3   D^{-1} L_I
-  static constexpr int O_PIV = O_Y + 24 * NA;  // NA (pivot rows, stored as doubles)
-  static constexpr int PER = O_PIV + NA;
+  static constexpr int POINT = O_CEA + 6 * NA;
+  // of the element: the points' shares [share][point], shares in the order f or K, L, D, R~
+  static constexpr int shares(bool want_k) { return (want_k ? 360 : 24) + 24 * NA + NT + NA; }
+  // after the points: T0^{-1} (GL), D, R~ and its solution, L, D^{-1} L, the row order
+  static constexpr int O_GEO = 8 * POINT;
+  static constexpr int O_D = O_GEO + 36;
+  static constexpr int O_RT = O_D + NA * NA;
+  static constexpr int O_L = O_RT + 2 * NA;    // NA x 24
+  static constexpr int O_Y = O_L + 24 * NA;    // 24 x NA
+  static constexpr int O_PERM = O_Y + 24 * NA; // NA
+  static constexpr int O_SHARE = O_PERM + NA;
+  static constexpr int total(bool want_k) { return O_SHARE + 8 * shares(want_k); }
 };
 
 __device__ __forceinline__ void packed_index(int t, int na, int& a, int& b) {
@@ -96,23 +107,20 @@ __device__ __forceinline__ void bop(const double F[3][3], const double dN[3], do
 }
 
 // HYP: the hyperelastic framework's material point (hyperelastic.cuh) instead of the closed-form laws
-template <int NA, int KIND, int MODE, typename KT, bool HYP>
-__global__ void __launch_bounds__(EasCfg<NA>::EPB * 8) eas_element_kernel(ElemArgs a, const int32_t* __restrict__ list,
-                                                                           int n_list, int e_base) {
+template <int NA, int KIND, int MODE, bool HYP>
+__global__ void __launch_bounds__(64) eas_element_kernel(ElemArgs a, const int32_t* __restrict__ list, int e_base) {
   using Cfg = EasCfg<NA>;
   constexpr bool WANT_R = MODE & kWantR;
   constexpr bool WANT_K = MODE & kWantK;
-  constexpr bool ELEM_OUT = MODE & kElemOut;
+  static_assert(WANT_R != WANT_K && (MODE & kElemOut), "element vectors or element matrices");
   extern __shared__ double smem[];
 
   const int lane = threadIdx.x & 31;
   const int sub = threadIdx.x & 7;
-  const int es = threadIdx.x >> 3;
-  double* sm = smem + (size_t)es * Cfg::PER;
-  const int li = blockIdx.x * Cfg::EPB + es;
-  const bool active = li < n_list;
-  const int lic = active ? li : n_list - 1;
-  const int e = list ? list[lic] : e_base + lic;
+  const int q = threadIdx.x >> 3;  // Gauss point
+  double* sm = smem + (size_t)q * Cfg::POINT;
+  const int li = blockIdx.x;
+  const int e = list ? list[li] : e_base + li;
   const int ne = a.n_elems;
   const int node = a.conn[sub * ne + e];
   const int src = lane & ~7;
@@ -132,7 +140,7 @@ __global__ void __launch_bounds__(EasCfg<NA>::EPB * 8) eas_element_kernel(ElemAr
   // centre data
   double A0[3][3] = {}, detJ0 = 0.0, dN0[3] = {0, 0, 0}, Fc0[3][3] = {}, Fa[3][3] = {};
   if (KIND == 1) {
-    for (int k = sub; k < 36; k += 8) sm[Cfg::O_GEO + k] = a.eas_geo[(size_t)k * ne + e];
+    if (threadIdx.x < 36) smem[Cfg::O_GEO + threadIdx.x] = a.eas_geo[(size_t)threadIdx.x * ne + e];
   } else {
 #pragma unroll
     for (int i = 0; i < 3; ++i)
@@ -152,29 +160,13 @@ __global__ void __launch_bounds__(EasCfg<NA>::EPB * 8) eas_element_kernel(ElemAr
         for (int c = 0; c < 3; ++c) Fa[i][c] = Fc0[i][0] * A0[0][c] + Fc0[i][1] * A0[1][c] + Fc0[i][2] * A0[2][c];
     }
   }
-  __syncwarp();
+  __syncthreads();
 
   const double lam = a.lam_e ? a.lam_e[e] : a.lam, mu = a.mu_e ? a.mu_e[e] : a.mu;
-  double f[3] = {0, 0, 0};
-  double Kacc[5][3][3];
-#pragma unroll
-  for (int d = 0; d < 5; ++d)
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-      for (int j = 0; j < 3; ++j) Kacc[d][i][j] = 0.0;
-  double Lacc[NA][3];
-#pragma unroll
-  for (int k = 0; k < NA; ++k) Lacc[k][0] = Lacc[k][1] = Lacc[k][2] = 0.0;
-  double Dacc[Cfg::DSH], Racc[Cfg::RSH];
-#pragma unroll
-  for (int m = 0; m < Cfg::DSH; ++m) Dacc[m] = 0.0;
-#pragma unroll
-  for (int m = 0; m < Cfg::RSH; ++m) Racc[m] = 0.0;
   int bad = 0;
-
-#pragma unroll 1
-  for (int q = 0; q < 8; ++q) {
+  double* share = smem + Cfg::O_SHARE + q;  // share t of this point at share[8 t]
+  constexpr int kL = WANT_K ? 360 : 24, kD = kL + 24 * NA, kR = kD + Cfg::NT;
+  {
     const double xi[3] = {(q & 1) ? kGaussHi : kGaussLo, (q & 2) ? kGaussHi : kGaussLo, (q & 4) ? kGaussHi : kGaussLo};
     double dxi[3];
     ref_gradient_at_gp<double>(sub, q, dxi);
@@ -252,7 +244,7 @@ __global__ void __launch_bounds__(EasCfg<NA>::EPB * 8) eas_element_kernel(ElemAr
         const double w = s[k] * al[k];
         const int rr = kRow[k];
 #pragma unroll
-        for (int r = 0; r < 6; ++r) Ev[r] += w * sm[Cfg::O_GEO + 6 * r + rr];
+        for (int r = 0; r < 6; ++r) Ev[r] += w * smem[Cfg::O_GEO + 6 * r + rr];
       }
     }
     double S[6], Sm[3][3];
@@ -355,7 +347,7 @@ __global__ void __launch_bounds__(EasCfg<NA>::EPB * 8) eas_element_kernel(ElemAr
         double t = 0.0;
 #pragma unroll
         for (int r = 0; r < 6; ++r) t += B[r][b] * S[r];
-        f[b] += w * t;
+        share[8 * (3 * sub + b)] = w * t;
       }
     }
     __syncwarp();  // C6 and dNm of all nodes are in shared memory
@@ -390,7 +382,7 @@ __global__ void __launch_bounds__(EasCfg<NA>::EPB * 8) eas_element_kernel(ElemAr
             double t = (i == j) ? kg : 0.0;
 #pragma unroll
             for (int r = 0; r < 6; ++r) t += V[r][i] * BJ[r][j];
-            Kacc[d][i][j] += w * t;
+            share[8 * ((d * 8 + sub) * 9 + 3 * i + j)] = w * t;
           }
       }
     }
@@ -400,7 +392,7 @@ __global__ void __launch_bounds__(EasCfg<NA>::EPB * 8) eas_element_kernel(ElemAr
       double Ea[6];
       if (KIND == 1) {
 #pragma unroll
-        for (int r = 0; r < 6; ++r) Ea[r] = s[k] * sm[Cfg::O_GEO + 6 * r + kRow[k]];
+        for (int r = 0; r < 6; ++r) Ea[r] = s[k] * smem[Cfg::O_GEO + 6 * r + kRow[k]];
       } else {
         const int r = k / 3, c = k % 3;
         double v[3], coef[3];
@@ -459,7 +451,7 @@ __global__ void __launch_bounds__(EasCfg<NA>::EPB * 8) eas_element_kernel(ElemAr
         }
       }
 #pragma unroll
-      for (int b = 0; b < 3; ++b) Lacc[k][b] += w * t[b];
+      for (int b = 0; b < 3; ++b) share[8 * (kL + 24 * k + 3 * sub + b)] = w * t[b];
     }
     // D share: (E_alpha^T C E_alpha + E_alpha,alpha) w detJ (enhancedassumedstrains.hh:400)
 #pragma unroll
@@ -486,7 +478,7 @@ __global__ void __launch_bounds__(EasCfg<NA>::EPB * 8) eas_element_kernel(ElemAr
           for (int i = 0; i < 3; ++i) Sfb[i] = Sm[i][0] * fb[0] + Sm[i][1] * fb[1] + Sm[i][2] * fb[2];
           x += (va[0] * vb[0] + va[1] * vb[1] + va[2] * vb[2]) * (fa[0] * Sfb[0] + fa[1] * Sfb[1] + fa[2] * Sfb[2]);
         }
-        Dacc[m] += w * x;
+        share[8 * (kD + t)] = w * x;
       }
     }
     // R~ share: E_alpha^T S w detJ (enhancedassumedstrains.hh:428)
@@ -497,216 +489,155 @@ __global__ void __launch_bounds__(EasCfg<NA>::EPB * 8) eas_element_kernel(ElemAr
         double x = 0.0;
 #pragma unroll
         for (int r = 0; r < 6; ++r) x += sm[Cfg::O_EA + 6 * k + r] * S[r];
-        Racc[m] += w * x;
+        share[8 * (kR + k)] = w * x;
       }
     }
-    __syncwarp();  // shared scratch is rewritten by the next Gauss point
   }
+  __syncthreads();
+
+  // ---- sums over the points, in their order ---------------------------------------------------------------
+  const double* shares = smem + Cfg::O_SHARE;
+  auto total = [&](int t) {
+    double x = shares[8 * t];
+#pragma unroll
+    for (int p = 1; p < 8; ++p) x += shares[8 * t + p];
+    return x;
+  };
+  double* L = smem + Cfg::O_L;
+  double* D = smem + Cfg::O_D;
+  double* Y = smem + Cfg::O_Y;
+  int* perm = reinterpret_cast<int*>(smem + Cfg::O_PERM);
+  for (int t = threadIdx.x; t < 24 * NA; t += 64) L[t] = total(kL + t);
+  for (int t = threadIdx.x; t < Cfg::NT; t += 64) {
+    int aa, bb;
+    packed_index(t, NA, aa, bb);
+    D[NA * aa + bb] = D[NA * bb + aa] = total(kD + t);
+  }
+  if (threadIdx.x < NA) {
+    smem[Cfg::O_RT + threadIdx.x] = total(kR + threadIdx.x);
+    perm[threadIdx.x] = threadIdx.x;
+  }
+  __syncthreads();
 
   // ---- static condensation ------------------------------------------------------------------------------
-#pragma unroll
-  for (int m = 0; m < Cfg::DSH; ++m) {
-    const int t = sub + 8 * m;
-    if (t < Cfg::NT) {
-      int aa, bb;
-      packed_index(t, NA, aa, bb);
-      sm[Cfg::O_D + NA * aa + bb] = Dacc[m];
-      sm[Cfg::O_D + NA * bb + aa] = Dacc[m];
-    }
-  }
-#pragma unroll
-  for (int m = 0; m < Cfg::RSH; ++m) {
-    const int k = sub + 8 * m;
-    if (k < NA) sm[Cfg::O_RT + k] = Racc[m];
-  }
-  __syncwarp();
-  if (sub == 0) {  // LU with partial pivoting of D in place
-    double* D = sm + Cfg::O_D;
+  if (threadIdx.x < 32) {
+    // LU with partial pivoting of D in place: lane i holds row i
     for (int k = 0; k < NA; ++k) {
-      int p = k;
-      double best = fabs(D[NA * k + k]);
-      for (int i = k + 1; i < NA; ++i)
-        if (fabs(D[NA * i + k]) > best) best = fabs(D[NA * i + k]), p = i;
-      sm[Cfg::O_PIV + k] = (double)p;
-      if (!(best > 0.0)) {
+      double best = lane >= k && lane < NA ? fabs(D[NA * lane + k]) : -1.0;
+      const bool nan = __any_sync(0xffffffffu, best != best);  // as a singular pivot, decided by all lanes alike
+      int p = lane;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {  // the largest, of equal ones the first row
+        const double v = __shfl_xor_sync(0xffffffffu, best, o);
+        const int w = __shfl_xor_sync(0xffffffffu, p, o);
+        if (v > best || (v == best && w < p)) best = v, p = w;
+      }
+      if (nan || !(best > 0.0)) {
         bad |= kStatusSingularD;
-        D[NA * k + k] = 1.0;
+        if (lane == 0) D[NA * k + k] = 1.0;
+        __syncwarp();
         continue;
       }
-      if (p != k)
-        for (int j = 0; j < NA; ++j) {
-          const double tmp = D[NA * k + j];
-          D[NA * k + j] = D[NA * p + j];
-          D[NA * p + j] = tmp;
-        }
-      const double inv = 1.0 / D[NA * k + k];
-      for (int i = k + 1; i < NA; ++i) {
-        const double l = D[NA * i + k] * inv;
-        D[NA * i + k] = l;
-        for (int j = k + 1; j < NA; ++j) D[NA * i + j] -= l * D[NA * k + j];
-      }
-    }
-  }
-  __syncwarp();
-  // solve D z = rhs with the factors (row swaps applied in order)
-  auto lu_solve = [&](double* z) {
-    const double* D = sm + Cfg::O_D;
-    for (int k = 0; k < NA; ++k) {
-      const int p = (int)sm[Cfg::O_PIV + k];
       if (p != k) {
-        const double t = z[k];
-        z[k] = z[p];
-        z[p] = t;
-      }
-    }
-    for (int i = 1; i < NA; ++i)
-      for (int j = 0; j < i; ++j) z[i] -= D[NA * i + j] * z[j];
-    for (int i = NA - 1; i >= 0; --i) {
-      for (int j = i + 1; j < NA; ++j) z[i] -= D[NA * i + j] * z[j];
-      z[i] /= D[NA * i + i];
-    }
-  };
-  double y[NA];
-#pragma unroll
-  for (int k = 0; k < NA; ++k) y[k] = sm[Cfg::O_RT + k];
-  lu_solve(y);
-#pragma unroll
-  for (int b = 0; b < 3; ++b) {
-    double z[NA];
-#pragma unroll
-    for (int k = 0; k < NA; ++k) z[k] = Lacc[k][b];
-    lu_solve(z);
-#pragma unroll
-    for (int k = 0; k < NA; ++k) sm[Cfg::O_Y + (3 * sub + b) * NA + k] = z[k];
-  }
-  __syncwarp();
-  if (WANT_R) {
-#pragma unroll
-    for (int b = 0; b < 3; ++b) {
-      double t = 0.0;
-#pragma unroll
-      for (int k = 0; k < NA; ++k) t += Lacc[k][b] * y[k];
-      f[b] -= t;
-    }
-  }
-  if (WANT_K) {
-#pragma unroll
-    for (int d = 0; d < 5; ++d) {
-      const int Jn = (sub + d) & 7;
-#pragma unroll
-      for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-          double t = 0.0;
-#pragma unroll
-          for (int k = 0; k < NA; ++k) t += Lacc[k][i] * sm[Cfg::O_Y + (3 * Jn + j) * NA + k];
-          Kacc[d][i][j] -= t;
+        if (lane < NA) {
+          const double t = D[NA * k + lane];
+          D[NA * k + lane] = D[NA * p + lane];
+          D[NA * p + lane] = t;
         }
+        if (lane == 0) {
+          const int t = perm[k];
+          perm[k] = perm[p];
+          perm[p] = t;
+        }
+        __syncwarp();
+      }
+      const double inv = 1.0 / D[NA * k + k];
+      if (lane > k && lane < NA) {
+        const double l = D[NA * lane + k] * inv;
+        D[NA * lane + k] = l;
+        for (int j = k + 1; j < NA; ++j) D[NA * lane + j] -= l * D[NA * k + j];
+      }
+      __syncwarp();
+    }
+    // columns of D^{-1} L (lanes 0 .. 23) and D^{-1} R~ (lane 24)
+    if (lane < 25) {
+      double z[NA];
+#pragma unroll
+      for (int k = 0; k < NA; ++k) z[k] = lane < 24 ? L[24 * perm[k] + lane] : smem[Cfg::O_RT + perm[k]];
+#pragma unroll
+      for (int i = 1; i < NA; ++i)
+#pragma unroll
+        for (int j = 0; j < i; ++j) z[i] -= D[NA * i + j] * z[j];
+#pragma unroll
+      for (int i = NA - 1; i >= 0; --i) {
+#pragma unroll
+        for (int j = i + 1; j < NA; ++j) z[i] -= D[NA * i + j] * z[j];
+        z[i] /= D[NA * i + i];
+      }
+      double* out = lane < 24 ? Y + lane * NA : smem + Cfg::O_RT + NA;
+#pragma unroll
+      for (int k = 0; k < NA; ++k) out[k] = z[k];
     }
   }
-
-  if (!active) return;
   if (bad && a.status) atomicOr(a.status, bad);
-  if (WANT_R && a.eas_y) {  // condensation cache for the state update
-    if (sub == 0)
-#pragma unroll
-      for (int k = 0; k < NA; ++k) a.eas_y[(size_t)k * ne + e] = y[k];
-#pragma unroll
-    for (int b = 0; b < 3; ++b)
-#pragma unroll
-      for (int k = 0; k < NA; ++k)
-        a.eas_Y[(size_t)(k * 24 + 3 * sub + b) * ne + e] = sm[Cfg::O_Y + (3 * sub + b) * NA + k];
-  }
-  const uint8_t fmaskI = a.node_fixed ? a.node_fixed[node] : uint8_t(0);
+  __syncthreads();
+
   if (WANT_R) {
-    if (a.trac_idx) {
-      const int t = a.trac_idx[e];
-      if (t >= 0)
-#pragma unroll
-        for (int c = 0; c < 3; ++c)
-          f[c] -= (a.load_factor_dev ? *a.load_factor_dev : a.load_factor) * a.trac[24 * t + 3 * sub + c];
+    const double* y = smem + Cfg::O_RT + NA;
+    if (a.eas_y) {  // condensation cache for the state update
+      if (threadIdx.x < NA) a.eas_y[(size_t)threadIdx.x * ne + e] = y[threadIdx.x];
+      for (int t = threadIdx.x; t < 24 * NA; t += 64) a.eas_Y[(size_t)t * ne + e] = Y[(t % 24) * NA + t / 24];
     }
-    if (a.ext) {
+    if (threadIdx.x < 24) {
+      const int i = threadIdx.x;
+      double f = total(i), t = 0.0;
 #pragma unroll
-      for (int c = 0; c < 3; ++c) f[c] -= a.ext[24 * (size_t)e + 3 * sub + c];
-    }
-    if (ELEM_OUT) {
-#pragma unroll
-      for (int c = 0; c < 3; ++c) a.elem_vec[24 * (size_t)li + 3 * sub + c] = f[c];
-    } else {
-#pragma unroll
-      for (int c = 0; c < 3; ++c)
-        if (!((fmaskI >> c) & 1)) a.R[3 * node + c] += f[c];
-    }
-  }
-  if (WANT_K) {
-    if (ELEM_OUT) {
-      double* out = a.elem_mat + 576 * (size_t)li;
-#pragma unroll
-      for (int d = 0; d < 5; ++d) {
-        const int Jn = (sub + d) & 7;
-#pragma unroll
-        for (int i = 0; i < 3; ++i)
-#pragma unroll
-          for (int j = 0; j < 3; ++j) {
-            out[(3 * Jn + j) * 24 + 3 * sub + i] = Kacc[d][i][j];
-            if (d >= 1 && d <= 3) out[(3 * sub + i) * 24 + 3 * Jn + j] = Kacc[d][i][j];
-          }
+      for (int k = 0; k < NA; ++k) t += L[24 * k + i] * y[k];
+      f -= t;
+      if (a.trac_idx) {
+        const int tr = a.trac_idx[e];
+        if (tr >= 0) f -= (a.load_factor_dev ? *a.load_factor_dev : a.load_factor) * a.trac[24 * tr + i];
       }
-    } else {
-      KT* val = static_cast<KT*>(a.Kval);
+      if (a.ext) f -= a.ext[24 * (size_t)e + i];
+      a.elem_vec[24 * (size_t)li + i] = f;
+    }
+  } else {
+    double* out = a.elem_mat + 576 * (size_t)li;
+    for (int t = threadIdx.x; t < 360; t += 64) {
+      const int d = t / 72, I = (t / 9) & 7, i = (t % 9) / 3, j = t % 3, J = (I + d) & 7;
+      double x = 0.0;
 #pragma unroll
-      for (int d = 0; d < 5; ++d) {
-        const int Jn = (sub + d) & 7;
-        const uint8_t fmaskJ = a.node_fixed ? a.node_fixed[a.conn[Jn * ne + e]] : uint8_t(0);
-        KT* b1 = val + block_entry(a.slot[(size_t)(sub * 8 + Jn) * ne + e], 0);  // entries 32 apart
-#pragma unroll
-        for (int i = 0; i < 3; ++i)
-#pragma unroll
-          for (int j = 0; j < 3; ++j)
-            if (!(((fmaskI >> i) | (fmaskJ >> j)) & 1)) b1[32 * (3 * i + j)] += KT(Kacc[d][i][j]);
-        if (d >= 1 && d <= 3) {
-          KT* b2 = val + block_entry(a.slot[(size_t)(Jn * 8 + sub) * ne + e], 0);
-#pragma unroll
-          for (int i = 0; i < 3; ++i)
-#pragma unroll
-            for (int j = 0; j < 3; ++j)
-              if (!(((fmaskI >> i) | (fmaskJ >> j)) & 1)) b2[32 * (3 * j + i)] += KT(Kacc[d][i][j]);
-        }
-      }
+      for (int k = 0; k < NA; ++k) x += L[24 * k + 3 * I + i] * Y[(3 * J + j) * NA + k];
+      const double v = total(t) - x;
+      out[(3 * J + j) * 24 + 3 * I + i] = v;
+      if (d >= 1 && d <= 3) out[(3 * I + i) * 24 + 3 * J + j] = v;
     }
   }
 }
 
-template <int NA, int KIND, int MODE, typename KT, bool HYP>
+template <int NA, int KIND, int MODE, bool HYP>
 void launch_t(const ElemArgs& a, const int32_t* list, int n_list, int e_base, cudaStream_t s) {
-  using Cfg = EasCfg<NA>;
-  const int blocks = (n_list + Cfg::EPB - 1) / Cfg::EPB;
-  const size_t shm = sizeof(double) * Cfg::PER * Cfg::EPB;
-  eas_element_kernel<NA, KIND, MODE, KT, HYP><<<blocks, Cfg::EPB * 8, shm, s>>>(a, list, n_list, e_base);
+  auto kern = eas_element_kernel<NA, KIND, MODE, HYP>;
+  constexpr int shm = (int)sizeof(double) * EasCfg<NA>::total(MODE & kWantK);
+  if (shm > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, shm);
+  kern<<<n_list, 64, shm, s>>>(a, list, e_base);
 }
 
+// element vectors or element matrices of the listed elements, in their order
 template <int NA, int KIND, bool HYP>
-void launch_kind(const ElemArgs& a, int mode, bool fp32, const int32_t* list, int n, int base, cudaStream_t s) {
-  switch (mode) {
-    case kWantR: launch_t<NA, KIND, kWantR, double, HYP>(a, list, n, base, s); break;
-    case kWantK:
-      if (fp32) launch_t<NA, KIND, kWantK, float, HYP>(a, list, n, base, s);
-      else launch_t<NA, KIND, kWantK, double, HYP>(a, list, n, base, s);
-      break;
-    case kWantR | kElemOut: launch_t<NA, KIND, kWantR | kElemOut, double, HYP>(a, list, n, base, s); break;
-    case kWantK | kElemOut: launch_t<NA, KIND, kWantK | kElemOut, double, HYP>(a, list, n, base, s); break;
-    default: break;
-  }
+void launch_kind(const ElemArgs& a, int mode, const int32_t* list, int n, int base, cudaStream_t s) {
+  if (mode == (kWantR | kElemOut)) launch_t<NA, KIND, kWantR | kElemOut, HYP>(a, list, n, base, s);
+  else if (mode == (kWantK | kElemOut)) launch_t<NA, KIND, kWantK | kElemOut, HYP>(a, list, n, base, s);
 }
 
 // the element launches of one material family (HYP: the hyperelastic framework)
 template <bool HYP>
-void launch_eas_family(const ElemArgs& a, int mode, bool fp32, const int32_t* list, int n, int base, cudaStream_t s) {
-  if (a.eas_kind == 1 && a.n_alpha == 9) launch_kind<9, 1, HYP>(a, mode, fp32, list, n, base, s);
-  else if (a.eas_kind == 1 && a.n_alpha == 21) launch_kind<21, 1, HYP>(a, mode, fp32, list, n, base, s);
-  else if (a.eas_kind == 2) launch_kind<9, 2, HYP>(a, mode, fp32, list, n, base, s);
-  else if (a.eas_kind == 3) launch_kind<9, 3, HYP>(a, mode, fp32, list, n, base, s);
+void launch_eas_family(const ElemArgs& a, int mode, const int32_t* list, int n, int base, cudaStream_t s) {
+  if (n <= 0) return;
+  if (a.eas_kind == 1 && a.n_alpha == 9) launch_kind<9, 1, HYP>(a, mode, list, n, base, s);
+  else if (a.eas_kind == 1 && a.n_alpha == 21) launch_kind<21, 1, HYP>(a, mode, list, n, base, s);
+  else if (a.eas_kind == 2) launch_kind<9, 2, HYP>(a, mode, list, n, base, s);
+  else if (a.eas_kind == 3) launch_kind<9, 3, HYP>(a, mode, list, n, base, s);
 }
 
 }  // namespace

@@ -6,9 +6,9 @@
 
 namespace ikr {
 
-void launch_eas_element_hyper(const ElemArgs& a, int mode, bool fp32, const int32_t* list, int n, int base,
+void launch_eas_element_hyper(const ElemArgs& a, int mode, const int32_t* list, int n, int base,
                               cudaStream_t s) {
-  launch_eas_family<true>(a, mode, fp32, list, n, base, s);
+  launch_eas_family<true>(a, mode, list, n, base, s);
 }
 
 }  // namespace ikr

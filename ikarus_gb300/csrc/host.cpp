@@ -113,25 +113,28 @@ void assemble_vector(ikr_asm a, ikr_req r, int dbc, bool sync) {
     f->refresh_function_loads(r->lambda);
   }
   a->R.alloc(a->n);
-  CK(cudaMemsetAsync(a->R.p, 0, sizeof(double) * a->n, f->stream));
+  f->build_node_corners();
   ikr::ElemArgs args = f->args();
   args.u = r->u.p;
   args.load_factor = r->lambda;
   args.load_factor_dev = sync ? nullptr : f->capture_lambda;
-  args.node_fixed = (dbc == IKR_DBC_RAW) ? nullptr : a->node_fixed.p;
-  args.R = a->R.p;
+  args.elem_vec = f->fel.p;
+  constexpr int kMode = ikr::kWantR | ikr::kElemOut;
   if (!f->epb_r) {
     f->epb_r = choose_epb(f, [&](int epb) {
-      CK(cudaMemsetAsync(a->R.p, 0, sizeof(double) * a->n, f->stream));
       ikr::ElemArgs t = args;
       t.epb = epb;
-      f->launch_coloured(t, ikr::kWantR, false);
+      f->launch_elements(t, kMode, false, nullptr, f->ne, 0);
       f->check_status();
     });
-    CK(cudaMemsetAsync(a->R.p, 0, sizeof(double) * a->n, f->stream));
   }
   args.epb = f->epb_r;
-  f->launch_coloured(args, ikr::kWantR, false);
+  // element forces, then every dof's sum over its elements in ascending order: two launches instead of one per colour,
+  // and no read-modify-write of R
+  f->launch_elements(args, kMode, false, nullptr, f->ne, 0);
+  ikr::launch_vector_gather(f->nc_ptr.p, f->nc_code.p, f->fel.p, dbc == IKR_DBC_RAW ? nullptr : a->node_fixed.p, f->nn,
+                            a->R.p, f->stream);
+  count(1);
   ikr::launch_vector_finish(a->R.p, nullptr, f->nn, a->pl_dof.p, a->pl_val.p, (int)a->pl_dof.n, r->lambda, f->stream,
                             args.load_factor_dev);
   if (a->pl_dof.n) count(1);
@@ -166,46 +169,36 @@ void assemble_matrix(ikr_asm a, ikr_req r, int dbc, bool sync) {
   ++a->k_stamp;
 }
 
-static void assemble_matrix_into(ikr_asm a, ikr_req r, int dbc, bool sync) {
+// FP32 displacement-based tangent
+static void assemble_matrix32(ikr_asm a, ikr::ElemArgs& args, const uint8_t* nf) {
   ikr_fes f = a->fes;
-  if (!a->nb) a->build_pattern();
-  const bool timed_path = a->fp32 && f->na == 0;  // the FP32 displacement tangent chooses its kernel by timing
-  if (!sync && !((a->fp32 ? f->epb_k32 : f->epb_k64) > 0 && (!timed_path || a->tan_path > 0)))
-    fail(IKR_ERR_INVALID_STATE, "tangent kernels not tuned before capture");
-  const uint8_t* nf = (dbc == IKR_DBC_RAW) ? nullptr : a->node_fixed.p;
-  ikr::ElemArgs args = f->args();
-  args.u = r->u.p;
-  args.load_factor = r->lambda;
-  args.node_fixed = nf;
-  args.Kval = a->values();
-  args.slot = a->slot.p;
-  int& epb_k = a->fp32 ? f->epb_k32 : f->epb_k64;
+  int& epb_k = f->epb_k32;
   if (!epb_k) {
     epb_k = choose_epb(f, [&](int epb) {
-      ikr::launch_bsr_reset(a->values(), a->fp32, a->npad, a->diag.p, nf, f->nn, f->stream);
+      ikr::launch_bsr_reset(a->values(), true, a->npad, a->diag.p, nf, f->nn, f->stream);
       ikr::ElemArgs t = args;
       t.epb = epb;
-      f->launch_coloured(t, ikr::kWantK, a->fp32);
+      f->launch_coloured(t, ikr::kWantK, true);
       f->check_status();
     });
-    ikr::launch_bsr_reset(a->values(), a->fp32, a->npad, a->diag.p, nf, f->nn, f->stream);
+    ikr::launch_bsr_reset(a->values(), true, a->npad, a->diag.p, nf, f->nn, f->stream);
   }
   args.epb = epb_k;
   // FP32 displacement-based tangent: the coloured element kernel, the row kernel (NeoHooke on one element set) or
   // element blocks + gather, whichever is fastest
-  const bool blocks_ok = a->fp32 && f->na == 0;
-  const bool row_ok = blocks_ok && f->material == 0 && f->n_inst == 0;
+  const bool row_ok = f->material == 0 && f->n_inst == 0;
   auto element_blocks = [&]() {
     a->build_gather_map();
+    a->eblk.alloc((size_t)f->ne * ikr::kElemBlockCount * 9);
     ikr::ElemArgs t = args;
     t.blk = a->eblk.p;
     f->launch_elements(t, ikr::kWantK | ikr::kElemBlocks, true, nullptr, f->ne, 0);
-    ikr::launch_tangent_gather(a->bsr(), a->gslice.p, a->inv_ptr.p, a->inv_idx.p, a->eblk.p, nf,
-                               static_cast<float*>(a->values()), f->stream);
+    ikr::launch_tangent_gather(a->bsr(), true, true, false, a->gslice.p, a->inv_ptr.p, a->inv_idx.p, a->eblk.p, nf,
+                               a->values(), f->stream);
     count(1);
   };
-  if (blocks_ok && a->tan_req && (a->tan_req != 2 || row_ok)) a->tan_path = a->tan_req;
-  if (blocks_ok && !a->tan_path) {
+  if (a->tan_req && (a->tan_req != 2 || row_ok)) a->tan_path = a->tan_req;
+  if (!a->tan_path) {
     cudaEvent_t e0, e1;
     CK(cudaEventCreate(&e0));
     CK(cudaEventCreate(&e1));
@@ -214,7 +207,7 @@ static void assemble_matrix_into(ikr_asm a, ikr_req r, int dbc, bool sync) {
       if (path == 2 && !row_ok) continue;
       float t = 1e30f;
       for (int rep = 0; rep < 2; ++rep) {
-        ikr::launch_bsr_reset(a->values(), a->fp32, a->npad, a->diag.p, nf, f->nn, f->stream);
+        ikr::launch_bsr_reset(a->values(), true, a->npad, a->diag.p, nf, f->nn, f->stream);
         CK(cudaEventRecord(e0, f->stream));
         if (path == 1) f->launch_coloured(args, ikr::kWantK, true);
         else if (path == 2) ikr::launch_row_tangent(args, a->ne_ptr.p, a->ne_elems.p, f->stream);
@@ -230,20 +223,51 @@ static void assemble_matrix_into(ikr_asm a, ikr_req r, int dbc, bool sync) {
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    ikr::launch_bsr_reset(a->values(), a->fp32, a->npad, a->diag.p, nf, f->nn, f->stream);
+    ikr::launch_bsr_reset(a->values(), true, a->npad, a->diag.p, nf, f->nn, f->stream);
   }
-  if (blocks_ok && a->tan_path == 3) {
+  if (a->tan_path == 3) {
     element_blocks();  // writes every entry of every slice, Dirichlet treatment included: no reset
   } else {
     // zero values, unit diagonal of the constrained dofs (Full), then the read-modify-write assembly
-    ikr::launch_bsr_reset(a->values(), a->fp32, a->npad, a->diag.p, nf, f->nn, f->stream);
+    ikr::launch_bsr_reset(a->values(), true, a->npad, a->diag.p, nf, f->nn, f->stream);
     count(1);
     if (row_ok && a->tan_path == 2) {
       ikr::launch_row_tangent(args, a->ne_ptr.p, a->ne_elems.p, f->stream);
       count(1);
     } else {
-      f->launch_coloured(args, ikr::kWantK, a->fp32);
+      f->launch_coloured(args, ikr::kWantK, true);
     }
+  }
+}
+
+static void assemble_matrix_into(ikr_asm a, ikr_req r, int dbc, bool sync) {
+  ikr_fes f = a->fes;
+  if (!a->nb) a->build_pattern();
+  const bool timed_path = a->fp32 && f->na == 0;  // the FP32 displacement tangent chooses its kernel by timing
+  if (!sync && !((a->fp32 ? f->epb_k32 : f->epb_k64) > 0 && (!timed_path || a->tan_path > 0)))
+    fail(IKR_ERR_INVALID_STATE, "tangent kernels not tuned before capture");
+  const uint8_t* nf = (dbc == IKR_DBC_RAW) ? nullptr : a->node_fixed.p;
+  ikr::ElemArgs args = f->args();
+  args.u = r->u.p;
+  args.load_factor = r->lambda;
+  args.node_fixed = nf;
+  args.Kval = a->values();
+  args.slot = a->slot.p;
+  const bool blocks32 = a->fp32 && f->na == 0;
+  if (!blocks32) {
+    // FP64 arithmetic: element blocks (displacement-based NeoHooke) or matrices of all elements, then every matrix
+    // block's sum in ascending element order with the Dirichlet treatment: two launches, no reset, no colouring
+    (a->fp32 ? f->epb_k32 : f->epb_k64) = 32;  // (these kernels have one launch shape)
+    a->build_gather_map();
+    const bool full = f->na > 0 || f->material != IKR_MATERIAL_NEOHOOKE;
+    a->eblk64.alloc((size_t)f->ne * (full ? 576 : ikr::kElemBlockCount * 9));
+    args.blk = args.elem_mat = a->eblk64.p;
+    f->launch_elements(args, ikr::kWantK | (full ? ikr::kElemOut : ikr::kElemBlocks), false, nullptr, f->ne, 0);
+    ikr::launch_tangent_gather(a->bsr(), a->fp32, false, full, a->gslice.p, a->inv_ptr.p, a->inv_idx.p, a->eblk64.p, nf,
+                               a->values(), f->stream);
+    count(1);
+  } else {
+    assemble_matrix32(a, args, nf);
   }
   if (a->me_idx.n) {  // AssemblerManipulator matrix hooks run after the Dirichlet treatment
     ikr::launch_add_entries(a->values(), a->fp32, a->me_idx.p, a->me_val.p, (int)a->me_idx.n, f->stream);

@@ -287,11 +287,27 @@ struct ikr_fes_s {
   }
 
   void launch_elements(const ikr::ElemArgs& a, int mode, bool fp32, const int32_t* list, int n, int base) {
-    if (na > 0) ikr::launch_eas_element(a, mode, fp32, list, n, base, stream);
+    if (na > 0) ikr::launch_eas_element(a, mode, list, n, base, stream);
     else ikr::launch_disp_element(a, mode, fp32, list, n, base, stream);
     count(1);
   }
-  // one launch per colour class: deterministic scatter without atomics
+  // element forces of all elements and the elements of every node (8 e + corner, ascending) they are gathered by
+  DBuf<double> fel;
+  DBuf<int32_t> nc_ptr, nc_code;
+  void build_node_corners() {
+    if (nc_code.p) return;
+    DBuf<int32_t> cnt, cursor;
+    cnt.alloc(nn), cursor.alloc(nn), nc_ptr.alloc(nn + 1);
+    ikr::launch_node_elem_count(conn.p, ne, nn, cnt.p, stream);
+    ikr::launch_exclusive_scan(cnt.p, nc_ptr.p, nn, stream);
+    fel.alloc(24 * (size_t)ne);
+    nc_code.alloc(8 * (size_t)ne);
+    ikr::launch_node_elem_fill(conn.p, ne, nc_ptr.p, cursor.p, nc_code.p, nn, stream);
+    ikr::launch_node_corners(conn.p, ne, nn, nc_ptr.p, nc_code.p, stream);
+    count(6);
+    CK(cudaStreamSynchronize(stream));
+  }
+  // one launch per colour class: deterministic scatter without atomics (the FP32 tangent's kernel 1)
   void launch_coloured(const ikr::ElemArgs& a, int mode, bool fp32) {
     for (size_t c = 0; c + 1 < colour_ptr.size(); ++c) {
       const int n = colour_ptr[c + 1] - colour_ptr[c];
@@ -332,16 +348,17 @@ struct ikr_asm_s {
   // FP32 tangent kernel: 0 = not chosen yet, 1 = coloured element kernel, 2 = row kernel, 3 = element blocks +
   // gather; req = forced choice
   int tan_path = 0, tan_req = 0;
-  // element blocks + gather: the FP32 blocks of every element, the inverse element-to-block map, the slice of every
-  // block column group
+  // gathered assembly: the blocks (FP32, FP64) or FP64 matrices of every element, the inverse element-to-block map, the
+  // slice of every block column group
   DBuf<float> eblk;
+  DBuf<double> eblk64;
   DBuf<int32_t> inv_ptr, inv_idx, gslice;
   void build_gather_map() {
     if (inv_idx.p) return;
     ikr_fes f = fes;
     cudaStream_t s = f->stream;
-    if (64LL * f->ne * ikr::kElemBlockCount * 2 >= (1LL << 31))
-      fail(IKR_ERR_NOT_IMPLEMENTED, "element-block tangent: too many elements for 32-bit block codes");
+    if (64LL * f->ne >= (1LL << 31))
+      fail(IKR_ERR_NOT_IMPLEMENTED, "gathered tangent: too many elements for 32-bit block codes");
     DBuf<int32_t> cnt, cursor;
     cnt.alloc(npad);
     cursor.alloc(npad);
@@ -357,7 +374,6 @@ struct ikr_asm_s {
     for (int sl = 0; sl < nslices; ++sl)
       for (int g = slice_off_h[sl]; g < slice_off_h[sl + 1]; ++g) gs[g] = sl;
     gslice.upload(gs.data(), gs.size(), s);
-    eblk.alloc((size_t)f->ne * ikr::kElemBlockCount * 9);
     CK(cudaStreamSynchronize(s));
   }
   DBuf<int32_t> row_ptr, col, diag, slot, slice_off, col_sell;

@@ -69,7 +69,6 @@ struct ElemArgs {
   double* eas_y = nullptr;         // cache: D^{-1} R~ (n_alpha x n_elems)
   double* eas_Y = nullptr;         // cache: D^{-1} L  (n_alpha*24 x n_elems)
   // outputs
-  double* R = nullptr;             // assembled residual (n dofs)
   void* Kval = nullptr;            // BSR values (float or double), 9 per block, row-major blocks
   const int32_t* slot = nullptr;   // 64 x n_elems: slot[(I*8+J) * n_elems + e] = BSR block of (node I, node J)
   double* elem_vec = nullptr;      // element-level: 24 per listed element
@@ -109,11 +108,10 @@ struct Bsr {
 // element.cu
 void launch_disp_element(const ElemArgs& a, int mode, bool fp32_tangent, const int32_t* list, int n_list, int e_base,
                          cudaStream_t s);
-void launch_eas_element(const ElemArgs& a, int mode, bool fp32_tangent, const int32_t* list, int n_list, int e_base,
-                        cudaStream_t s);
+// EAS elements: kWantR | kElemOut or kWantK | kElemOut (element vectors or matrices)
+void launch_eas_element(const ElemArgs& a, int mode, const int32_t* list, int n_list, int e_base, cudaStream_t s);
 // element_eas_hyper.cu: the same for material 3 (the hyperelastic framework)
-void launch_eas_element_hyper(const ElemArgs& a, int mode, bool fp32_tangent, const int32_t* list, int n_list,
-                              int e_base, cudaStream_t s);
+void launch_eas_element_hyper(const ElemArgs& a, int mode, const int32_t* list, int n_list, int e_base, cudaStream_t s);
 // the element's stored block of corner pair (I, J) for kElemBlocks, as (index p << 1) | transposed
 __host__ __device__ __forceinline__ int tangent_block_code(int I, int J) {
   const int d = (J - I) & 7;
@@ -122,14 +120,22 @@ __host__ __device__ __forceinline__ int tangent_block_code(int I, int J) {
   return ((8 * (8 - d) + J) << 1) | 1;  // (J, I) is stored, transposed
 }
 constexpr int kElemBlockCount = 36;
-// gathered FP32 tangent assembly (element.cu): inverse of the element-to-block map -- for every padded block id the
-// element blocks that add to it, (e * 36 + p) << 1 | transposed, ascending -- and the gather that sums them, applies
-// the Full Dirichlet treatment (node_fixed; unit diagonal) and writes every entry of every slice once
+// gathered tangent assembly (element.cu): inverse of the element-to-block map -- for every padded block id the element
+// blocks that add to it, e * 64 + 8 I + J for the corner pair (I, J), ascending -- and the gather that sums them, applies
+// the Full Dirichlet treatment (node_fixed; unit diagonal) and writes every entry of every slice once.  blk: the 36
+// distinct blocks of every element (FP32 or FP64), or with `full` FP64 24 x 24 column-major matrices.
 void launch_tangent_inverse_count(const int32_t* slot, int n_elems, int32_t* cnt, cudaStream_t s);
 void launch_tangent_inverse_fill(const int32_t* slot, int n_elems, const int32_t* ptr, int32_t* cursor, int32_t* inv,
                                  int64_t n_padded, cudaStream_t s);
-void launch_tangent_gather(const Bsr& A, const int32_t* gslice, const int32_t* inv_ptr, const int32_t* inv,
-                           const float* blk, const uint8_t* node_fixed, float* val, cudaStream_t s);
+void launch_tangent_gather(const Bsr& A, bool fp32_val, bool fp32_blk, bool full, const int32_t* gslice,
+                           const int32_t* inv_ptr, const int32_t* inv, const void* blk, const uint8_t* node_fixed,
+                           void* val, cudaStream_t s);
+// gathered residual assembly: the elements of every node (ascending, from launch_node_elem_fill) as 8 e + corner, and R
+// of every dof as the sum of its elements' forces vec (24 per element), zero where node_fixed says so
+void launch_node_corners(const int32_t* conn, int n_elems, int n_nodes, const int32_t* ptr, int32_t* codes,
+                         cudaStream_t s);
+void launch_vector_gather(const int32_t* ptr, const int32_t* codes, const double* vec, const uint8_t* node_fixed,
+                          int n_nodes, double* R, cudaStream_t s);
 // displacement-based NeoHooke FP32 tangent by block rows (thread per node row, no colouring; element.cu);
 // ne_ptr / ne_elems: the elements of every node in ascending order
 void launch_row_tangent(const ElemArgs& a, const int32_t* ne_ptr, const int32_t* ne_elems, cudaStream_t s);
