@@ -423,7 +423,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1) pcg_halo_kernel(const __grid_co
 
   while (done == 0) {
     const uint32_t tag = (uint32_t)it + 1u;
-    // ---- p of the own rows first: the neighbours wait for it; then the sums r.z and r.r of the new vectors
+    // ---- p of the own rows first: the neighbours wait for it
 #pragma unroll
     for (int j = 0; j < MAXP; ++j) {
       if (MAXP > 1 && j * WARPS * kRowsPerWarp >= m) break;
@@ -441,6 +441,29 @@ __global__ void __launch_bounds__(WARPS * 32, 1) pcg_halo_kernel(const __grid_co
         }
       }
     }
+    // ---- halo: every row once, polled until it carries this iteration's tag; without a stream (registers) the first
+    // batch's reads travel while the sums are formed
+    T vx[kBatch], vy[kBatch], vz[kBatch];
+    unsigned pend = 0;
+    auto fetch = [&](int i0) {
+#pragma unroll
+      for (int j = 0; j < kBatch; ++j)
+        if ((pend >> j) & 1u)
+          if (fetch_row(H.p, hl[i0 + j * kThreads], tag, vx[j], vy[j], vz[j])) pend &= ~(1u << j);
+    };
+    auto wanted = [&](int i0) {
+#pragma unroll
+      for (int j = 0; j < kBatch; ++j)
+        if (i0 + j * kThreads < nh) pend |= 1u << j;
+    };
+    wait_cycles(kPollDelay);
+    wanted(tid);
+    bool got[kBatch];
+#pragma unroll
+    for (int j = 0; j < kBatch; ++j) {
+      got[j] = false;
+      if (!STREAM && ((pend >> j) & 1u)) got[j] = fetch_row(H.p, hl[tid + j * kThreads], tag, vx[j], vy[j], vz[j]);
+    }
     if (warp < nwr) {
       T srz = T(0), srr = T(0);
 #pragma unroll
@@ -452,24 +475,19 @@ __global__ void __launch_bounds__(WARPS * 32, 1) pcg_halo_kernel(const __grid_co
         }
       warp_parts<T>(srz, srr, T(0), &swS[3][warp], &swx[3][warp], WARPS);
     }
-    wait_cycles(kPollDelay);
-    // ---- halo: every row once, polled until it carries this iteration's tag
+#pragma unroll
+    for (int j = 0; j < kBatch; ++j)
+      if (got[j]) pend &= ~(1u << j);
 #pragma unroll 1
     for (int i0 = tid; i0 < nh; i0 += kBatch * kThreads) {
-      T vx[kBatch], vy[kBatch], vz[kBatch];
-      unsigned pend = 0;
-#pragma unroll
-      for (int j = 0; j < kBatch; ++j)
-        if (i0 + j * kThreads < nh) pend |= 1u << j;
+      if (i0 != tid) wanted(i0);
 #pragma unroll 1
       for (int k = 0; pend && k < H.wc.polls; ++k) {
         if (k > 64) __nanosleep(16);
-#pragma unroll
-        for (int j = 0; j < kBatch; ++j)
-          if ((pend >> j) & 1u)
-            if (fetch_row(H.p, hl[i0 + j * kThreads], tag, vx[j], vy[j], vz[j])) pend &= ~(1u << j);
+        fetch(i0);
       }
       if (pend) failed = true;
+      pend = 0;
 #pragma unroll
       for (int j = 0; j < kBatch; ++j) {
         const int i = i0 + j * kThreads;
