@@ -14,11 +14,12 @@
 //             P^T r; the CTA that finishes last sums the chunks of every aggregate in a fixed order (r_c), forms
 //             e = A_c^-1 r_c with the dense inverse, r.z = r.D^-1 r + r_c.e, and beta (or the initial r.z);
 //   prolong:  z += P e.
-// Setup per tangent (A_c): for every colour of a distance-2 colouring of the aggregates, the six probe vectors
-// sum_{a of that colour} P_{a,m} are multiplied by K (launch_spmv64) and restricted per chunk (36 sums); the
-// host adds the chunks of each aggregate in a fixed order, places each block at the single aggregate of the
-// colour that touches it, and inverts A_c (ikr_ls_s in host_internal.h).  All sums are fixed-order: results are
-// bit-identical run to run.
+// Setup per tangent (A_c): one pass over the matrix.  A block K_IJ of rows in aggregate b and columns in aggregate b + d
+// (|d| <= reach) adds P_I^T K_IJ P_J to A_c(b, b + d); a thread sums W = sum_J K_IJ P_J of its row per d (27 FP64
+// instructions per block, the translations being additions), then P_I^T W, a CTA its 256 rows, and a second kernel the
+// CTAs of an aggregate in order.  The host symmetrises A_c and inverts it (ikr_ls_s in host_internal.h).  All sums are
+// fixed-order: results are bit-identical run to run.  Measured at 140 481 rows, three distances: 18 probe products
+// K V_m (164 us each, the matrix read 18 times) and their restrictions took 3.3 ms, this pass 0.83 ms.
 #include "cg_common.cuh"
 
 namespace ikr {
@@ -148,49 +149,73 @@ __global__ void __launch_bounds__(256) coarse_prolong_kernel(Coarse C, T* z, con
   }
 }
 
-// probe vectors of one colour: V_m (dof-major FP64, m = 0..5, stride 3 n_rows) = P_{a,m} on the nodes of every
-// aggregate a of that colour, zero elsewhere
-__global__ void coarse_probe_kernel(Coarse C, int colour, double* __restrict__ V) {
-  const int64_t stride = 3LL * C.n_rows;
-  for (int node = blockIdx.x * blockDim.x + threadIdx.x; node < C.n_rows; node += gridDim.x * blockDim.x) {
-    const NodeP n = node_p(C.y4, node);
-    const bool on = __ldg(C.agg_colour + n.agg) == colour;
-    double P[3][6];
-    p_cols(n, P);
+constexpr int kGalerkinRows = 256;
+// part[((d + reach) * n_parts + part) * 36 + 6 r + m], one CTA per run of kGalerkinRows nodes of a chunk
+template <typename T>
+__global__ void __launch_bounds__(kGalerkinRows) coarse_galerkin_kernel(Coarse C, Bsr A, const T* __restrict__ val,
+                                                                        int reach, int runs, double* __restrict__ part) {
+  __shared__ double sh[kGalerkinRows / 32][36];
+  const int chunk = blockIdx.x / runs, run = blockIdx.x - chunk * runs;
+  const int i = C.chunk_off[chunk] + run * kGalerkinRows + threadIdx.x;
+  const bool active = i < C.chunk_off[chunk + 1];
+  const int node = active ? __ldg(C.nodes + i) : 0;
+  const NodeP n = node_p(C.y4, node);
+  double P[3][6];
+  p_cols(n, P);
+  const int g0 = A.slice_off[node >> 5], width = active ? A.slice_off[(node >> 5) + 1] - g0 : 0, l = node & 31;
+  for (int d = -reach; d <= reach; ++d) {
+    double W[3][6] = {};
+    bool any = false;
+    for (int k = 0; k < width; ++k) {
+      const int J = __ldg(A.col_sell + 32 * (int64_t)(g0 + k) + l);
+      const NodeP nj = node_p(C.y4, J);
+      if (nj.agg != n.agg + d) continue;
+      any = true;
+      const T* v = val + (int64_t)(g0 + k) * 288 + l;
+      const double y0 = nj.y[0], y1 = nj.y[1], y2 = nj.y[2];
+      const bool m0 = nj.mask & 1, m1 = nj.mask & 2, m2 = nj.mask & 4;
 #pragma unroll
-    for (int m = 0; m < 6; ++m)
+      for (int c = 0; c < 3; ++c) {
+        const double a0 = m0 ? double(__ldg(v + 96 * c)) : 0.0, a1 = m1 ? double(__ldg(v + 96 * c + 32)) : 0.0,
+                     a2 = m2 ? double(__ldg(v + 96 * c + 64)) : 0.0;
+        W[c][0] += a0, W[c][1] += a1, W[c][2] += a2;
+        W[c][3] = fma(a2, y1, fma(-a1, y2, W[c][3]));  // e_k x y
+        W[c][4] = fma(a0, y2, fma(-a2, y0, W[c][4]));
+        W[c][5] = fma(a1, y0, fma(-a0, y1, W[c][5]));
+      }
+    }
+    double* out = part + ((size_t)(d + reach) * gridDim.x + blockIdx.x) * 36;
+    if (!__syncthreads_or(any)) {  // no row of this run couples with aggregate b + d
+      if (threadIdx.x < 36) out[threadIdx.x] = 0.0;
+      continue;
+    }
 #pragma unroll
-      for (int c = 0; c < 3; ++c) V[m * stride + 3 * node + c] = on ? P[c][m] : 0.0;
+    for (int r = 0; r < 6; ++r)
+#pragma unroll
+      for (int m = 0; m < 6; ++m) {
+        const double t = warp_sum(P[0][r] * W[0][m] + P[1][r] * W[1][m] + P[2][r] * W[2][m]);
+        if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5][6 * r + m] = t;
+      }
+    __syncthreads();
+    if (threadIdx.x < 36) {
+      double t = 0.0;
+#pragma unroll
+      for (int w = 0; w < kGalerkinRows / 32; ++w) t += sh[w][threadIdx.x];
+      out[threadIdx.x] = t;
+    }
+    __syncthreads();
   }
 }
-
-// 36 sums per chunk: part[36 k + 6 r + m] = sum over the chunk's nodes of P[:, r] . W_m
-__global__ void __launch_bounds__(256) coarse_galerkin_kernel(Coarse C, const double* __restrict__ W,
-                                                              double* __restrict__ part) {
-  __shared__ double sh[32];
-  const int64_t stride = 3LL * C.n_rows;
-  const int k = blockIdx.x;
-  double s[36];
-#pragma unroll
-  for (int q = 0; q < 36; ++q) s[q] = 0.0;
-  for (int i = C.chunk_off[k] + threadIdx.x; i < C.chunk_off[k + 1]; i += blockDim.x) {
-    const int node = __ldg(C.nodes + i);
-    const NodeP n = node_p(C.y4, node);
-    double P[3][6];
-    p_cols(n, P);
-#pragma unroll
-    for (int m = 0; m < 6; ++m) {
-      const double w0 = __ldg(W + m * stride + 3 * node), w1 = __ldg(W + m * stride + 3 * node + 1),
-                   w2 = __ldg(W + m * stride + 3 * node + 2);
-#pragma unroll
-      for (int r = 0; r < 6; ++r) s[6 * r + m] += P[0][r] * w0 + P[1][r] * w1 + P[2][r] * w2;
-    }
-  }
-#pragma unroll
-  for (int q = 0; q < 36; ++q) {
-    const double t = block_sum_all(s[q], sh);
-    if (threadIdx.x == 0) part[36 * k + q] = t;
-  }
+// blk[((d + reach) * n_agg + b) * 36 + q]: the runs of aggregate b in order
+__global__ void coarse_blocks_kernel(Coarse C, int nd, int runs, const double* __restrict__ part,
+                                     double* __restrict__ blk) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= nd * C.n_agg * 36) return;
+  const int q = t % 36, b = t / 36 % C.n_agg, d = t / 36 / C.n_agg;
+  double s = 0.0;
+  const size_t n_parts = (size_t)C.n_chunks * runs;
+  for (int k = C.agg_chunk[b] * runs; k < C.agg_chunk[b + 1] * runs; ++k) s += part[(d * n_parts + k) * 36 + q];
+  blk[t] = s;
 }
 
 int grid_for(int n, int bs, int cap) {
@@ -209,11 +234,14 @@ void launch_coarse_correction(const Coarse& C, const PcgWork& w, bool init, cuda
     coarse_prolong_kernel<double><<<w.grid, 256, 0, s>>>(C, (double*)w.z, w.scal);
   }
 }
-void launch_coarse_probe(const Coarse& C, int colour, double* V, cudaStream_t s) {
-  coarse_probe_kernel<<<grid_for(C.n_rows, 256, 1216), 256, 0, s>>>(C, colour, V);
-}
-void launch_coarse_galerkin(const Coarse& C, const double* W, double* part, cudaStream_t s) {
-  coarse_galerkin_kernel<<<C.n_chunks, 256, 0, s>>>(C, W, part);
+int coarse_galerkin_runs(int chunk_rows) { return (chunk_rows + kGalerkinRows - 1) / kGalerkinRows; }
+void launch_coarse_galerkin(const Coarse& C, const Bsr& A, bool fp32, int reach, int runs, double* part, double* blk,
+                            cudaStream_t s) {
+  const int grid = C.n_chunks * runs;
+  if (fp32) coarse_galerkin_kernel<float><<<grid, kGalerkinRows, 0, s>>>(C, A, (const float*)A.val, reach, runs, part);
+  else coarse_galerkin_kernel<double><<<grid, kGalerkinRows, 0, s>>>(C, A, (const double*)A.val, reach, runs, part);
+  const int nd = 2 * reach + 1;
+  coarse_blocks_kernel<<<(nd * C.n_agg * 36 + 127) / 128, 128, 0, s>>>(C, nd, runs, part, blk);
 }
 
 }  // namespace ikr

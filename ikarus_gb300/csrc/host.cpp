@@ -793,8 +793,37 @@ int ikr_assembler_matrix(ikr_asm a, ikr_req r, int32_t aff, int32_t dbc) {
 
 static void export_csc(ikr_asm a, int dbc, int64_t* cp, int32_t* ri, double* v, int64_t* nnz_out) {
   need(a && a->nb, IKR_ERR_INVALID_STATE, "no matrix assembled");
-  const bool reduced = dbc == IKR_DBC_REDUCED;
   const int nn = a->fes->nn;
+  if (dbc != IKR_DBC_REDUCED) {
+    // every block is present as 3 x 3 scalars: counts follow from the pattern, indices and values are expanded on the
+    // device in their final order.  4 225 nodes (0.9 M entries): 5.8 ms of
+    // host loops -> 0.47 ms with the copies
+    const int64_t nnz = 9 * a->nb;
+    if (cp)
+      for (int J = 0; J < nn; ++J)
+        for (int b = 0; b < 3; ++b)
+          cp[3 * J + b] = 9LL * a->row_ptr_h[J] + 3LL * b * (a->row_ptr_h[J + 1] - a->row_ptr_h[J]);
+    if (cp) cp[3 * nn] = nnz;
+    // through a staging buffer of at most a million blocks, kept with the assembler
+    constexpr int64_t kStage = 1 << 20;
+    const auto& rp = a->row_ptr_h;
+    for (int J0 = 0, J1 = 0; (ri || v) && J0 < nn; J0 = J1) {
+      J1 = J0 + 1;
+      while (J1 < nn && rp[J1 + 1] - rp[J0] <= kStage) ++J1;
+      const int64_t n = 9LL * (rp[J1] - rp[J0]), at = 9LL * rp[J0];
+      if (ri && (int64_t)a->csc_ri.n < n) a->csc_ri.alloc(n);
+      if (v && (int64_t)a->csc_v.n < n) a->csc_v.alloc(n);
+      ikr::launch_export_csc(a->bsr(), a->fp32, J0, J1, ri ? a->csc_ri.p : nullptr, v ? a->csc_v.p : nullptr,
+                             a->fes->stream);
+      count(1);
+      CK(cudaGetLastError());
+      if (ri) a->csc_ri.download(ri + at, n, a->fes->stream);
+      if (v) a->csc_v.download(v + at, n, a->fes->stream);
+      CK(cudaStreamSynchronize(a->fes->stream));
+    }
+    if (nnz_out) *nnz_out = nnz;
+    return;
+  }
   std::vector<double> val;
   if (v) {
     val.resize(9 * (size_t)a->npad);
@@ -823,13 +852,13 @@ static void export_csc(ikr_asm a, int dbc, int64_t* cp, int32_t* ri, double* v, 
   for (int J = 0; J < nn; ++J)
     for (int b = 0; b < 3; ++b) {
       const int gc = 3 * J + b;
-      if (reduced && a->fixed_h[gc]) continue;
+      if (a->fixed_h[gc]) continue;
       for (int k = rp[J]; k < rp[J + 1]; ++k) {
         const int I = cl[k];
         for (int aa = 0; aa < 3; ++aa) {
           const int gr = 3 * I + aa;
-          if (reduced && a->fixed_h[gr]) continue;
-          if (ri) ri[nnz] = reduced ? gr - a->cb_h[gr] : gr;
+          if (a->fixed_h[gr]) continue;
+          if (ri) ri[nnz] = gr - a->cb_h[gr];
           if (v) v[nnz] = val[ikr::block_entry(block_of(I, J), 3 * aa + b)];
           ++nnz;
         }

@@ -397,6 +397,8 @@ struct ikr_asm_s {
   std::map<std::pair<int32_t, int32_t>, double> me_h;
   DBuf<int64_t> me_idx;
   DBuf<double> me_val;
+  DBuf<int32_t> csc_ri;  // staging of the CSC export
+  DBuf<double> csc_v;
   DBuf<double> norm_part, norm_out;
   ikr_req bound_req = nullptr;
   int bound_dbc = IKR_DBC_FULL;
@@ -545,11 +547,11 @@ struct ikr_ls_s {
     int n_slabs = 0, reach = 0, n_colours = 0, dropped = 0;
     ikr::Coarse C;
     DBuf<float> y4;
-    DBuf<int32_t> nodes, chunk_off, agg_chunk, agg_colour;
+    DBuf<int32_t> nodes, chunk_off, agg_chunk;
     std::vector<int32_t> agg_chunk_h;
-    DBuf<double> rpart, gpart, V, W, ainv64, e64, cpart;
+    DBuf<double> rpart, gpart, gblk, ainv64, e64, cpart;
     DBuf<float> ainv32, e32;
-    std::vector<double> gpart_h, ac, inv, fac;
+    std::vector<double> gblk_h, ac, inv, fac;
     std::vector<float> inv32;
   } co;
   DBuf<double> dx2, dr2, dz2, dp2, dp12, pa2, pb2, pbi2, scal2;
@@ -746,6 +748,7 @@ struct ikr_ls_s {
 
   // ---- coarse correction: aggregates, A_c = P^T K P and its inverse (coarse.cu has the device side) ----
 
+  static constexpr int kCoarseChunk = 2048;  // nodes of an aggregate per CTA of the restriction
   // slab aggregates and the per-node mode data, once per assembler and slab count
   void coarse_layout(ikr_asm a) {
     ikr_fes f = a->fes;
@@ -800,15 +803,12 @@ struct ikr_ls_s {
       fail(IKR_ERR_ARG, "coarse correction: slabs thinner than the elements couple %d slabs apart; use fewer slabs",
            reach);
     const int ncol = std::min(2 * reach + 1, S);
-    std::vector<int32_t> colour(S);
-    for (int a_ = 0; a_ < S; ++a_) colour[a_] = a_ % ncol;
     // chunks of at most 2048 nodes per aggregate: one 1024-thread CTA of the restrict kernel each, one CTA per SM
     // (its registers), so about as many chunks as SMs keep the launch in one wave
-    constexpr int kChunk = 2048;
     std::vector<int32_t> chunk_off{0};
     co.agg_chunk_h.assign(1, 0);
     for (int a_ = 0; a_ < S; ++a_) {
-      for (int k = agg_off[a_]; k < agg_off[a_ + 1]; k += kChunk) chunk_off.push_back(std::min(k + kChunk, agg_off[a_ + 1]));
+      for (int k = agg_off[a_]; k < agg_off[a_ + 1]; k += kCoarseChunk) chunk_off.push_back(std::min(k + kCoarseChunk, agg_off[a_ + 1]));
       co.agg_chunk_h.push_back((int32_t)chunk_off.size() - 1);
     }
     const int nchunks = (int)chunk_off.size() - 1;
@@ -816,7 +816,6 @@ struct ikr_ls_s {
     co.nodes.upload(order.data(), order.size(), s);
     co.chunk_off.upload(chunk_off.data(), chunk_off.size(), s);
     co.agg_chunk.upload(co.agg_chunk_h.data(), co.agg_chunk_h.size(), s);
-    co.agg_colour.upload(colour.data(), colour.size(), s);
     co.rpart.alloc(6 * (size_t)nchunks);
     const size_t nc = 6 * (size_t)S;
     if (fp32) co.ainv32.alloc(nc * nc), co.e32.alloc(nc);
@@ -824,7 +823,7 @@ struct ikr_ls_s {
     ikr::Coarse& C = co.C;
     C.n_rows = nn, C.n_agg = S, C.n_c = (int)nc, C.n_chunks = nchunks;
     C.y4 = reinterpret_cast<const float4*>(co.y4.p);
-    C.nodes = co.nodes.p, C.chunk_off = co.chunk_off.p, C.agg_chunk = co.agg_chunk.p, C.agg_colour = co.agg_colour.p;
+    C.nodes = co.nodes.p, C.chunk_off = co.chunk_off.p, C.agg_chunk = co.agg_chunk.p;
     C.rpart = co.rpart.p;
     C.ainv = fp32 ? (const void*)co.ainv32.p : (const void*)co.ainv64.p;
     C.e = fp32 ? (void*)co.e32.p : (void*)co.e64.p;
@@ -832,7 +831,7 @@ struct ikr_ls_s {
     co.built_for = a, co.n_slabs = S, co.reach = reach, co.n_colours = ncol;
   }
 
-  // A_c = P^T K P from probe products (one SpMV per colour and mode), then its inverse
+  // A_c = P^T K P in one pass over the tangent, then its inverse
   void coarse_operator(ikr_asm a) {
     if (co.built_for != a || co.n_slabs != std::min(coarse_req, a->fes->nn) ||
         (fp32 ? (const void*)co.ainv32.p : (const void*)co.ainv64.p) != co.C.ainv) {
@@ -845,35 +844,24 @@ struct ikr_ls_s {
     co.since_rebuild = 0;
     cudaStream_t s = a->fes->stream;
     const ikr::Bsr A = a->bsr();
-    const int S = co.n_slabs, nc = 6 * S, nch = co.C.n_chunks, ncol = co.n_colours;
+    const int S = co.n_slabs, nc = 6 * S, nch = co.C.n_chunks;
     co.cpart.alloc(2 * (size_t)(nc + 2) * w.grid);  // partials of the fused coarse CG (parity, CTA, coarse dof)
     w.coarse_part = co.cpart.p;
     w.coarse_part_ctas = w.grid;
-    const int64_t n3 = 3LL * a->fes->nn;
-    co.V.alloc(6 * (size_t)n3), co.W.alloc(6 * (size_t)n3);
-    co.gpart.alloc(36 * (size_t)nch * ncol);
-    for (int c = 0; c < ncol; ++c) {
-      ikr::launch_coarse_probe(co.C, c, co.V.p, s);
-      for (int m = 0; m < 6; ++m) ikr::launch_spmv64(A, fp32, co.V.p + m * n3, co.W.p + m * n3, s);
-      ikr::launch_coarse_galerkin(co.C, co.W.p, co.gpart.p + 36LL * nch * c, s);
-      count(8);
-    }
-    co.gpart_h.resize(co.gpart.n);
-    co.gpart.download(co.gpart_h.data(), co.gpart.n, s);
+    const int runs = ikr::coarse_galerkin_runs(kCoarseChunk), nd = 2 * co.reach + 1;
+    co.gpart.alloc(36 * (size_t)nch * runs * nd);
+    co.gblk.alloc(36 * (size_t)S * nd);
+    ikr::launch_coarse_galerkin(co.C, A, fp32, co.reach, runs, co.gpart.p, co.gblk.p, s);
+    count(2);
+    co.gblk_h.resize(co.gblk.n);
+    co.gblk.download(co.gblk_h.data(), co.gblk.n, s);
     CK(cudaStreamSynchronize(s));
-    // the blocks: row aggregate b, column aggregate = the one aggregate of colour c within reach of b
     co.ac.assign((size_t)nc * nc, 0.0);
-    for (int c = 0; c < ncol; ++c)
-      for (int b = 0; b < S; ++b) {
-        int col_agg = -1;
-        for (int d = -co.reach; d <= co.reach; ++d)
-          if (b + d >= 0 && b + d < S && (b + d) % ncol == c) col_agg = b + d;
-        if (col_agg < 0) continue;
-        double blk[36] = {};
-        for (int k = co.agg_chunk_h[b]; k < co.agg_chunk_h[b + 1]; ++k)
-          for (int q = 0; q < 36; ++q) blk[q] += co.gpart_h[36 * ((size_t)nch * c + k) + q];
+    for (int d = -co.reach; d <= co.reach; ++d)
+      for (int b = std::max(0, -d); b < std::min(S, S - d); ++b) {
+        const double* blk = co.gblk_h.data() + 36 * ((size_t)(d + co.reach) * S + b);
         for (int r = 0; r < 6; ++r)
-          for (int m = 0; m < 6; ++m) co.ac[(size_t)(6 * b + r) * nc + 6 * col_agg + m] = blk[6 * r + m];
+          for (int m = 0; m < 6; ++m) co.ac[(size_t)(6 * b + r) * nc + 6 * (b + d) + m] = blk[6 * r + m];
       }
     for (int i = 0; i < nc; ++i)
       for (int j = 0; j < i; ++j) {

@@ -179,6 +179,8 @@ void launch_slot_map(const int32_t* conn, int n_elems, const int32_t* row_ptr, c
                      const int32_t* slice_off, int32_t* slot, int32_t* diag, int n_nodes, cudaStream_t s);
 void launch_bsr_reset(void* val, bool fp32, int64_t n_padded, const int32_t* diag, const uint8_t* node_fixed,
                       int n_nodes, cudaStream_t s);
+// the scalar CSC of block columns [J0, J1) in column order: row indices and / or values (either may be null)
+void launch_export_csc(const Bsr& A, bool fp32, int J0, int J1, int32_t* ri, double* v, cudaStream_t s);
 // val[idx[k]] += v[k] for n unique value indices (the assembler manipulator's matrix entries)
 void launch_add_entries(void* val, bool fp32, const int64_t* idx, const double* v, int n, cudaStream_t s);
 void launch_vector_finish(double* R, const uint8_t* node_fixed, int n_nodes, const int32_t* pl_dof,
@@ -286,7 +288,6 @@ struct Coarse {
   const int32_t* nodes = nullptr;      // node ids grouped by aggregate
   const int32_t* chunk_off = nullptr;  // nodes of chunk k: nodes[chunk_off[k] .. chunk_off[k+1])
   const int32_t* agg_chunk = nullptr;  // chunks of aggregate a: [agg_chunk[a], agg_chunk[a+1])
-  const int32_t* agg_colour = nullptr; // colour of every aggregate (distance-2 colouring)
   double* rpart = nullptr;             // 6 per chunk: P^T r of the chunk
   const void* ainv = nullptr;          // A_c^-1, n_c x n_c in the CG's type
   void* e = nullptr;                   // A_c^-1 P^T r, n_c in the CG's type
@@ -298,8 +299,11 @@ constexpr int kCoarseFusedMaxDofs = 384;
 int pcg_coarse_variants();
 bool pcg_coarse_eligible(const Bsr& A, PcgWork& w, const Coarse& C, int variant);
 cudaError_t launch_pcg_coarse(const Bsr& A, PcgWork& w, const Coarse& C, int variant, cudaStream_t s);
-void launch_coarse_probe(const Coarse& C, int colour, double* V, cudaStream_t s);
-void launch_coarse_galerkin(const Coarse& C, const double* W, double* part, cudaStream_t s);
+// A_c in blocks: blk[((d + reach) n_agg + b) 36 + 6 r + m] of the aggregate pair (b, b + d); part holds 36 doubles per
+// distance, chunk and run (coarse_galerkin_runs of the largest chunk)
+int coarse_galerkin_runs(int chunk_rows);
+void launch_coarse_galerkin(const Coarse& C, const Bsr& A, bool fp32, int reach, int runs, double* part, double* blk,
+                            cudaStream_t s);
 int pcg_persistent_variants();
 bool pcg_persistent_eligible(const Bsr& A, PcgWork& w, int variant);
 // cg_halo.cu -- the last kHaloVariants persistent variants where the system has a split that fits

@@ -315,6 +315,42 @@ void launch_bsr_reset(void* val, bool fp32, int64_t n_padded, const int32_t* dia
   if (fp32) unit_diag_kernel<float><<<blocks_for(n_nodes, 256), 256, 0, s>>>((float*)val, diag, node_fixed, n_nodes);
   else unit_diag_kernel<double><<<blocks_for(n_nodes, 256), 256, 0, s>>>((double*)val, diag, node_fixed, n_nodes);
 }
+// Scalar CSC of block columns [J0, J1) (Eigen's column-major layout), from the first of them on: one thread per block
+// (I, J) of block column J, which by the pattern's symmetry is entry k of block row J.  Column 3 J + b starts at 9 row_ptr[J] + 3 b len(J) and holds the rows
+// 3 I + a of every neighbour I in ascending order; K(3 I + a, 3 J + b) sits in block (I, J) of block row I.
+template <typename T>
+__global__ void export_csc_kernel(const int32_t* __restrict__ row_ptr, const int32_t* __restrict__ col,
+                                  const int32_t* __restrict__ slice_off, const T* __restrict__ val, int J0, int J1,
+                                  int32_t* __restrict__ ri, double* __restrict__ v) {
+  // a warp per block column: its lanes take neighbours, so a column's entries are written side by side
+  const int J = J0 + (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+  if (J >= J1) return;
+  const int k0 = row_ptr[J], len = row_ptr[J + 1] - k0;
+  for (int k = lane; k < len; k += 32) {
+    const int I = col[k0 + k];
+    const int64_t base = 9LL * (k0 - row_ptr[J0]) + 3 * k;
+    if (ri)
+#pragma unroll
+      for (int b = 0; b < 3; ++b)
+#pragma unroll
+        for (int a = 0; a < 3; ++a) ri[base + 3LL * b * len + a] = 3 * I + a;
+    if (v) {
+      const int r0 = row_ptr[I];
+      const int64_t id = block_id(slice_off, I, find_col(col, r0, row_ptr[I + 1], J) - r0);
+#pragma unroll
+      for (int b = 0; b < 3; ++b)
+#pragma unroll
+        for (int a = 0; a < 3; ++a) v[base + 3LL * b * len + a] = double(val[block_entry(id, 3 * a + b)]);
+    }
+  }
+}
+void launch_export_csc(const Bsr& A, bool fp32, int J0, int J1, int32_t* ri, double* v, cudaStream_t s) {
+  if (J1 <= J0) return;
+  const int blocks = blocks_for(32LL * (J1 - J0), 256);
+  if (fp32) export_csc_kernel<float><<<blocks, 256, 0, s>>>(A.row_ptr, A.col, A.slice_off, (const float*)A.val, J0, J1, ri, v);
+  else export_csc_kernel<double><<<blocks, 256, 0, s>>>(A.row_ptr, A.col, A.slice_off, (const double*)A.val, J0, J1, ri, v);
+}
+
 // AssemblerManipulator matrix entries: val[idx[k]] += v[k] (indices unique, so no two threads touch one value)
 template <typename T>
 __global__ void add_entries_kernel(T* __restrict__ val, const int64_t* __restrict__ idx, const double* __restrict__ v,
