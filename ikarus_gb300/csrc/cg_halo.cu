@@ -23,8 +23,8 @@
 //     total is as good as one of doubles; it does not depend on an order.
 // Measured, microseconds per iteration, the best of the two-barrier forms -> this kernel:
 //   rows        44            425           2 673         18 785        35 721        140 481
-//   FP32   10.3 ->  3.6  13.6 ->  4.3  13.9 ->  4.4  14.2 ->  6.2  14.5 ->  8.2  29.7 -> 24.5
-//   FP64   16.3 ->  4.7  36.1 ->  5.5  38.9 ->  7.0  39.8 -> 15.7  39.8 -> 26.1   128 ->   79
+//   FP32   10.3 ->  3.6  13.6 ->  4.1  13.9 ->  4.4  14.2 ->  6.0  14.5 ->  7.9  29.7 -> 23.3
+//   FP64   16.3 ->  4.7  36.1 ->  5.5  38.9 ->  7.0  39.8 -> 15.0  39.8 -> 24.3   128 ->   77
 // The small sizes are bound by two trips through L2 (p to the neighbours, the sums to everyone) and the chains between
 // them, FP64 from 18 785 rows on by the FP64 pipe (nine multiply-adds per block: 8, 15 and 54 us of the last three), FP32
 // at 140 481 rows by the 152 MB of blocks streamed through L2.
@@ -53,7 +53,7 @@ constexpr int kSmemBudget = 224 * 1024;
 // FP32 3.37 / 3.54 / 3.61 / 3.70 (eleven CTAs, hardly any skew), 425 rows 4.62 / 4.41 / 4.29 / 4.22, 18 785 rows 6.36 /
 // 6.28 / 6.22 / 6.20, 140 481 rows 25.9 / 26.0 / 26.0 / 26.1.
 constexpr int kPollDelay = 450;
-constexpr int kMaxRing = 4;  // stages of streamed block columns per warp
+constexpr int kMaxRing = 2;  // stages of streamed block columns per warp
 template <typename T>
 constexpr int unit_bytes() {
   return 288 * (int)sizeof(T) + 64;  // nine entries and a 16-bit local column of 32 lanes
@@ -234,7 +234,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1) pcg_halo_kernel(const __grid_co
   constexpr int NC = STREAM ? 3 : 1;  // components of a row that a lane holds
   constexpr int kRowsPerWarp = rows_per_warp(STREAM);
   // the inverse blocks of a lane's rows in registers where the register file allows it
-  constexpr bool kRegM = MAXP * NC * sizeof(T) <= 48;
+  constexpr bool kRegM = MAXP * NC * sizeof(T) <= 24;
   constexpr int kBatch = STREAM ? 4 : 2;  // halo rows a thread fetches at a time (6: 1.4 us slower at 140 481 rows)
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(8) uint64_t bars[WARPS][STREAM ? kMaxRing : 1];
@@ -391,14 +391,16 @@ __global__ void __launch_bounds__(WARPS * 32, 1) pcg_halo_kernel(const __grid_co
     mbar_init_fence();
   }
   __syncwarp();
+  const uint32_t keep16 = (uint32_t)(65536.0 * 32.0 * (double)H.keep_g / (double)A.n_padded);
   auto issue = [&](int st, int u) {
     if (lane == 0) {
       const int64_t g = g0 + u;
       const uint32_t b = smem_addr(&bars[warp][st]);
       const uint32_t nb = min(kUnits, ue - u);
       unsigned char* d = ring + (size_t)st * kUnits * kUnitBytes;
-      // the share kept in L2 is the same of every warp's run
-      const uint64_t pol = l2_policy((int64_t)(u - ures) * A.n_padded < H.keep_g * 32 * (int64_t)(ue - ures));
+      // the stages kept in L2 are spread over the run (a low-discrepancy sequence), so that reads from DRAM and from L2
+      // overlap: with the kept ones first, an iteration at 140 481 rows FP32 took 25.3 us, so 23.3
+      const uint64_t pol = l2_policy((((uint32_t)((u - ures) / kUnits) * 2654435769u) >> 16) < keep16);
       mbar_expect_tx(b, nb * kUnitBytes);
       bulk_g2s(smem_addr(d), H.val + g * 288, nb * kValBytes, b, pol);
       bulk_g2s(smem_addr(d + kUnits * kValBytes), P.col16 + g * 32, nb * kColBytes, b, pol);
@@ -810,13 +812,13 @@ Layout layout_of(const HaloPlan& P, int warps) {
     L.resident = per;
     L.passes = passes(false);
   } else {
-    // stages in flight first, as the bandwidth of the stream comes from them (about 150 KB per SM in FP32); FP64 is
-    // bound by its arithmetic and keeps more columns resident
+    // two stages in flight first, as the bandwidth of the stream comes from them: four block columns each in FP32 (two:
+    // 13.2 instead of 10.0 us per iteration at 60 625 rows, although more columns stay resident), two in FP64 (one: 26.1
+    // instead of 24.8 us at 35 721 rows), less where the vectors leave no room
     L.passes = passes(true);
     if (P.chunk < 32 || L.passes > 4) return L;
-    L.units = sizeof(T) == 8 ? 1 : units >= 8 && L.passes <= 2 ? 4 : 2;
-    L.ring = sizeof(T) == 8 ? 3 : L.units == 4 ? 2 : 3;
-    while (L.ring > 2 && L.ring * L.units > units) --L.ring;
+    L.units = sizeof(T) == 8 ? (units >= 4 ? 2 : 1) : units >= 8 && L.passes <= 2 ? 4 : 2;
+    L.ring = 2;
     if (L.ring * L.units > units) return L;
     L.resident = std::min(units - L.ring * L.units, per);
   }
@@ -859,8 +861,9 @@ cudaError_t launch_variant(const Bsr& A, PcgWork& w, const Layout& L, cudaStream
   return cudaLaunchCooperativeKernel((const void*)kern, dim3(H.P.n_cta), dim3(WARPS * 32), args, L.bytes, s);
 }
 
-// warps per CTA of a variant.  Variant 0 is the one that measured faster: FP32 16 (8: 0.3 us faster per iteration below
-// 5000 rows, 0.6 us slower at 18 785), FP64 8 (16 spill and are no faster: the FP64 pipe is the bound)
+// warps per CTA of a variant; the tuner times both where both exist.  FP32 16 (8: 0.1 us faster per iteration below 5 000
+// rows, 0.3 us slower at 18 785 and not built for streams), FP64 8 (16: slower below 20 000 rows, 3 % faster at 35 721,
+// 9 % at 60 625)
 constexpr int warps_of(bool fp32, int variant) { return fp32 == (variant == 0) ? 16 : 8; }
 
 cudaError_t launch(const Bsr& A, PcgWork& w, int variant, cudaStream_t s) {
@@ -875,11 +878,15 @@ cudaError_t launch(const Bsr& A, PcgWork& w, int variant, cudaStream_t s) {
   }
   const Layout L = layout_of<double>(*w.halo, warps_of(false, variant));
   if (!L.ok) return cudaErrorInvalidConfiguration;
-  if (variant == 1)
-    return L.ring ? launch_variant<double, 16, 2, 1>(A, w, L, s) : launch_variant<double, 16, 2, 0>(A, w, L, s);
+  if (variant == 1) {
+    if (!L.ring) return launch_variant<double, 16, 2, 0>(A, w, L, s);
+    if (L.units == 1) return launch_variant<double, 16, 2, 1>(A, w, L, s);
+    return L.passes <= 1 ? launch_variant<double, 16, 1, 2>(A, w, L, s) : launch_variant<double, 16, 2, 2>(A, w, L, s);
+  }
   if (!L.ring) return L.passes <= 1 ? launch_variant<double, 8, 1, 0>(A, w, L, s) : launch_variant<double, 8, 2, 0>(A, w, L, s);
-  if (L.passes <= 1) return launch_variant<double, 8, 1, 1>(A, w, L, s);
-  return L.passes <= 2 ? launch_variant<double, 8, 2, 1>(A, w, L, s) : launch_variant<double, 8, 4, 1>(A, w, L, s);
+  if (L.units == 1) return launch_variant<double, 8, 4, 1>(A, w, L, s);
+  if (L.passes <= 1) return launch_variant<double, 8, 1, 2>(A, w, L, s);
+  return L.passes <= 2 ? launch_variant<double, 8, 2, 2>(A, w, L, s) : launch_variant<double, 8, 4, 2>(A, w, L, s);
 }
 // variant 1 exists where it can be faster: FP32 without a stream, FP64 up to two passes
 Layout usable(const PcgWork& w, int variant) {
