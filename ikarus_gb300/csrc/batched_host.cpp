@@ -84,13 +84,15 @@ BatchChoice choose_batch_plan(const std::vector<int>& rows, const std::vector<in
   return out;
 }
 
-// CTA groups of one batched CG launch over the instances in `run` (choose_batch_plan on the device's co-resident
-// capacities, a share of them while another solver's batched CG runs concurrently); largest instances first.
-static void plan_batch_launch(ikr_nr nr, ikr_fes f, ikr_asm a, bool fp32, const std::vector<int>& run) {
+// The planner's choice over the instances in `run`, on the device's co-resident capacities (a share of them while
+// another solver's batched CG runs concurrently); order: largest instances first.
+static BatchChoice planned(ikr_nr nr, ikr_fes f, ikr_asm a, bool fp32, const std::vector<int>& run,
+                           std::vector<int>& order) {
   auto& P = nr->plan;
   const int sms = num_sms();
   const int nr_ = (int)run.size();
-  std::vector<int> rows(nr_), width(nr_, 0), order(nr_);
+  std::vector<int> rows(nr_), width(nr_, 0);
+  order.resize(nr_);
   for (int k = 0; k < nr_; ++k) {
     const int r0 = f->inst_off_h[run[k]], r1 = f->inst_off_h[run[k] + 1];
     rows[k] = r1 - r0, order[k] = k;
@@ -101,8 +103,15 @@ static void plan_batch_launch(ikr_nr nr, ikr_fes f, ikr_asm a, bool fp32, const 
   auto share = [&](int cap) { return std::max(1, (int)(cap * P.share)); };
   int caps[6];
   for (int v = 0; v < 6; ++v) caps[v] = v == 4 ? 0 : share(ikr::batched_pcg_capacity(fp32, v, sms));
-  const BatchChoice ch =
-      choose_batch_plan(rows, width, fp32, P.variant, caps, fp32 ? share(ikr::batched_cluster_capacity()) : 0);
+  return choose_batch_plan(rows, width, fp32, P.variant, caps, fp32 ? share(ikr::batched_cluster_capacity()) : 0);
+}
+
+// CTA groups of one batched CG launch over the instances in `run`.
+static void plan_batch_launch(ikr_nr nr, ikr_fes f, ikr_asm a, bool fp32, const std::vector<int>& run) {
+  auto& P = nr->plan;
+  const int sms = num_sms();
+  std::vector<int> order;
+  const BatchChoice ch = planned(nr, f, a, fp32, run, order);
   std::vector<int32_t> ci, cf, cs;
   if (ch.variant == 4) {  // one cluster per instance: the kernel takes the instance of each cluster
     for (int k : order) ci.push_back(run[k]);
@@ -130,8 +139,61 @@ static void plan_batch_launch(ikr_nr nr, ikr_fes f, ikr_asm a, bool fp32, const 
   }
 }
 
+// CTA groups of one launch of the one-reduction kernel (cg_halo.cu): one CTA per SM; an instance gets as many as the
+// smallest number of slices per CTA allows at which all groups fit.  False where there are more instances than SMs or a
+// CTA's share does not fit its registers and shared memory (more than 2 048 rows per CTA in FP32, 1 024 in FP64; the
+// halo is bounded by the instance, so that the launch needs no answer from the device: instances of more than about
+// 9 000 and 6 000 rows).  Instances that leave a solve only make the shares of the others smaller.
+static bool plan_halo_launch(ikr_nr nr, ikr_fes f, ikr_asm a, bool fp32, const std::vector<int>& run) {
+  auto& P = nr->plan;
+  const int n = (int)run.size(), cap = std::min(num_sms(), 160);
+  if (n > cap) return false;
+  std::vector<int> order(run);
+  auto rows = [&](int i) { return f->inst_off_h[i + 1] - f->inst_off_h[i]; };
+  auto slice_a = [&](int i) { return f->inst_off_h[i] >> 5; };
+  auto slices = [&](int i) { return ((f->inst_off_h[i + 1] - 1) >> 5) - slice_a(i) + 1; };
+  std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return rows(x) > rows(y); });
+  int lo = 1, hi = slices(order[0]) + 1;  // the slices of the instance with the most rows, one more at most
+  while (lo < hi) {
+    const int q = (lo + hi) / 2;
+    int64_t t = 0;
+    for (int i : run) t += (slices(i) + q - 1) / q;
+    if (t <= cap) hi = q;
+    else lo = q + 1;
+  }
+  ikr::HaloPlan S;
+  std::vector<int32_t> ci, cf, cs;
+  P.max_rows = rows(order[0]);
+  for (int i : order) {
+    const int ns = slices(i), g = (ns + lo - 1) / lo, first = (int)ci.size(), sa = slice_a(i);
+    for (int k = 0; k < g; ++k) {
+      ci.push_back(i), cf.push_back(first), cs.push_back(g);
+      const int s0 = sa + (int)((int64_t)k * ns / g), s1 = sa + (int)((int64_t)(k + 1) * ns / g);
+      const int own = std::min(f->inst_off_h[i + 1], 32 * s1) - std::max(f->inst_off_h[i], 32 * s0);
+      S.max_ns = std::max(S.max_ns, s1 - s0);
+      S.max_units = std::max(S.max_units, a->slice_off_h[s1] - a->slice_off_h[s0]);
+      S.max_halo = std::max(S.max_halo, rows(i) - own);
+    }
+  }
+  S.n_cta = (int)ci.size();
+  S.halo_cap = S.max_halo;
+  if (!ikr::batched_halo_fits(S, fp32)) return false;
+  cudaStream_t s = f->stream;
+  for (auto* b : {&P.cta_inst, &P.cta_first, &P.cta_size, &P.halo_cnt})
+    if (b->n < (size_t)cap) b->alloc(cap);
+  if (P.halo_rows.n < (size_t)S.n_cta * S.halo_cap) P.halo_rows.alloc((size_t)S.n_cta * S.halo_cap);
+  if (P.col16.n < (size_t)a->bsr().n_padded) P.col16.alloc(a->bsr().n_padded);
+  S.halo_cnt = P.halo_cnt.p, S.halo = P.halo_rows.p, S.col16 = P.col16.p;
+  P.halo_split = S;
+  P.n_cta = S.n_cta;
+  CK(cudaMemcpyAsync(P.cta_inst.p, ci.data(), sizeof(int32_t) * ci.size(), cudaMemcpyHostToDevice, s));
+  CK(cudaMemcpyAsync(P.cta_first.p, cf.data(), sizeof(int32_t) * cf.size(), cudaMemcpyHostToDevice, s));
+  CK(cudaMemcpyAsync(P.cta_size.p, cs.data(), sizeof(int32_t) * cs.size(), cudaMemcpyHostToDevice, s));
+  return true;
+}
+
 // The batched CG of one Newton iteration: the instances with act set start their PCG on -R; the solve runs as a
-// sequence of launches of 128, 256, ... (at most 4096) iterations, each re-planned over the instances still
+// sequence of launches of 128, 256, ... (at most 4096, or 256) iterations, each re-planned over the instances still
 // running, so that the hard instances that outlast the others get more CTAs and one row per thread.  Instances not
 // in the solve get a zero correction.  cgit: CG iterations per instance (0 for those not in the solve).
 static void batched_cg(ikr_nr nr, ikr_fes f, ikr_asm a, const std::vector<uint8_t>& act, std::vector<int32_t>& cgit) {
@@ -152,9 +214,28 @@ static void batched_cg(ikr_nr nr, ikr_fes f, ikr_asm a, const std::vector<uint8_
   std::vector<int32_t> flag(ni), its(ni);
   int chunk = std::max(1, P.first_chunk);
   bool first = true;
+  // the planner's own choice runs as the one-reduction kernel where that fits and no other solver shares the device; the
+  // launches count as the planner's variant
+  const bool halo = P.variant == -1 && P.share >= 1.0 && plan_halo_launch(nr, f, a, a->fp32, run);
+  // the one-reduction kernel is re-planned more often: the CTAs of finished instances idle until the launch ends, which
+  // at six microseconds per iteration costs more than a launch (128 instances, FP32: 119 / 117 / 121 / 123 ms at most
+  // 128 / 256 / 512 / 1 024 iterations; 100 instances, FP64: 380 / 383 / 397 / 397 ms)
+  const int longest = halo ? 256 : 4096;
   while (!run.empty()) {
-    plan_batch_launch(nr, f, a, a->fp32, run);
-    if (P.cur_variant == 4)
+    if (halo) {
+      std::vector<int> order;
+      P.cur_variant = planned(nr, f, a, a->fp32, run, order).variant;
+      need(first || plan_halo_launch(nr, f, a, a->fp32, run), IKR_ERR_ARG, "the batched CG's split does not fit");
+    } else {
+      plan_batch_launch(nr, f, a, a->fp32, run);
+    }
+    if (halo) {
+      CK(ikr::launch_batched_halo(a->bsr(), w, P.halo_split, P.halo_cnt.p, P.halo_rows.p, P.col16.p, P.max_rows,
+                                  nr->rhs.p, nr->corr.p, f->inst_off.p, P.cta_inst.p, P.cta_first.p, P.cta_size.p,
+                                  nr->inst_rtol.p, st.linear_max_iter, chunk, first, P.st.p, nr->inst_cg_iters.p,
+                                  P.flag.p, ni, nr->inst_cg_res.p, s));
+      count(first ? 2 : 1);
+    } else if (P.cur_variant == 4)
       CK(ikr::launch_batched_pcg_cluster(a->bsr(), w.minv, nr->rhs.p, nr->corr.p, P.n_cta, f->inst_off.p,
                                          P.cta_inst.p, w.x, w.r, w.z, w.p0, w.p1, nr->inst_rtol.p, st.linear_max_iter,
                                          chunk, first ? 1 : 0, P.st.p, nr->inst_cg_iters.p, P.flag.p,
@@ -169,7 +250,7 @@ static void batched_cg(ikr_nr nr, ikr_fes f, ikr_asm a, const std::vector<uint8_
     ++P.launches;
     ++P.launches_by_variant[P.cur_variant];
     first = false;
-    chunk = std::min(2 * chunk, std::max(chunk, 4096));
+    chunk = std::min(2 * chunk, std::max(chunk, longest));
     P.flag.download(flag.data(), ni, s);
     CK(cudaStreamSynchronize(s));
     std::vector<int> next;

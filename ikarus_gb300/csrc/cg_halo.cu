@@ -28,6 +28,8 @@
 // The small sizes are bound by two trips through L2 (p to the neighbours, the sums to everyone) and the chains between
 // them, FP64 from 18 785 rows on by the FP64 pipe (nine multiply-adds per block: 8, 15 and 54 us of the last three), FP32
 // at 140 481 rows by the 152 MB of blocks streamed through L2.
+// GROUPS: the same for many independent instances, a group of CTAs each (plan_halo_launch in batched_host.cpp).  A load
+// step of 128 instances in mixed precision 227 -> 117 ms, of 100 in FP64 819 -> 383 ms against the kernels of batched.cu.
 // The launch is cooperative (all CTAs co-resident) and every wait is bounded: one that gives up ends the CTA with
 // scal[kDone] = 6 after its copies in flight have been drained, and with it the waits of the others.
 #include <algorithm>
@@ -146,10 +148,15 @@ __device__ __noinline__ Num warp_sum(long long m, int x) {
 }
 // Warp sums of three values at once (the redux chains overlap), as S * 2^x with |S| < 2^62, to slot `warp` of the CTA's
 // lists S[k * stride], x[k * stride]
-template <typename T>
+// (PAIR: the second value is v1 + v2, v2 below a unit in the last place of v1, and there is no third)
+template <typename T, bool PAIR = false>
 __device__ __noinline__ void warp_parts(T v0, T v1, T v2, long long* S, int* x, int stride) {
   __syncwarp();
-  const Num u[3] = {num_of(v0), num_of(v1), num_of(v2)};
+  Num u[3] = {num_of(v0), num_of(v1), num_of(v2)};
+  if (PAIR) {
+    u[1].S += shift_right(u[2].S, u[1].x - u[2].x);
+    u[2] = {0, kZeroExp};
+  }
   int X[3];
   uint32_t lo[3], mid[3];
   int hi[3];
@@ -199,6 +206,28 @@ __device__ __forceinline__ double reciprocal(double d) {
   return y;
 }
 
+// Independent instances of one element set, a group of CTAs each (the GROUPS form of the kernel): CTA b is number
+// b - first[b] of the size[b] that serve instance inst[b], whose rows are [node_off[inst], node_off[inst + 1]).  The slices
+// an instance's rows touch are split evenly over its group; lanes of other instances' rows compute along unseen.
+struct HaloGroups {
+  const int32_t *inst, *first, *size, *node_off;
+  const double* rtol;  // per instance
+  int max_iter, chunk;  // an instance's iterations in all and in one launch
+  void* p;              // p between the launches of a solve (node-padded)
+  double* st;           // four per instance, the third b.b
+  int32_t *its, *flag;
+  double *relres, *x_out;
+};
+struct GroupRows {
+  int s0, ns, lo, hi;  // slices and rows [lo, hi) of a CTA
+};
+__device__ __forceinline__ GroupRows group_rows(const HaloGroups& g, int b) {
+  const int i = g.inst[b], r0 = g.node_off[i], r1 = g.node_off[i + 1], sa = r0 >> 5, n = ((r1 - 1) >> 5) - sa + 1;
+  const int k = b - g.first[b], m = g.size[b];
+  const int a = sa + (int)((int64_t)k * n / m), e = sa + (int)((int64_t)(k + 1) * n / m);
+  return {a, e - a, max(r0, 32 * a), min(r1, 32 * e)};
+}
+
 template <typename T>
 struct HaloArgs {
   HaloPlan P;
@@ -216,6 +245,7 @@ struct HaloArgs {
   // shared memory: elements of a p component and of a component of the partial products, resident block columns per
   // warp, stages of the stream per warp
   int np, qstride, resident, ring;
+  HaloGroups g;
 };
 
 // Who owns a row in the vector part of an iteration.  Small systems (CB = 0): warps in tens of rows, lane 3 k + c holding
@@ -225,7 +255,7 @@ constexpr int rows_per_warp(bool streamed) { return streamed ? 32 : 10; }
 
 // CB: streamed block columns per stage; 0: everything is resident and the code of the stream is left out, which keeps
 // the loop body of the latency-bound sizes small.
-template <typename T, int WARPS, int MAXP, int CB>
+template <typename T, int WARPS, int MAXP, int CB, bool GROUPS>
 __global__ void __launch_bounds__(WARPS * 32, 1) pcg_halo_kernel(const __grid_constant__ HaloArgs<T> H) {
   constexpr int kThreads = WARPS * 32;
   constexpr int kValBytes = 288 * (int)sizeof(T), kColBytes = 64, kUnitBytes = unit_bytes<T>();
@@ -248,8 +278,9 @@ __global__ void __launch_bounds__(WARPS * 32, 1) pcg_halo_kernel(const __grid_co
   const HaloPlan& P = H.P;
   const Bsr& A = H.A;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int G = gridDim.x, cta = blockIdx.x;
-  const int ch = P.chunk;
+  const int G = GROUPS ? H.g.size[blockIdx.x] : gridDim.x, cta = GROUPS ? blockIdx.x - H.g.first[blockIdx.x] : blockIdx.x;
+  const int ch = GROUPS ? 32 : P.chunk;
+  double* part = GROUPS ? H.part + 2 * H.g.first[blockIdx.x] : H.part;
 
   // layout: units (resident, then the ring), p components, partial products, halo rows, slice offsets
   const int resident = H.resident;
@@ -265,8 +296,15 @@ __global__ void __launch_bounds__(WARPS * 32, 1) pcg_halo_kernel(const __grid_co
   int* soff = hl + P.max_halo;
 
   // own rows [row0, row0 + m), slices [s0, s0 + ns), units (block columns, or chunks of them) [0, ng)
-  int row0, m, s0, ns, ng;
-  if (ch == 32) {
+  // (GROUPS: the rows start at row0 + off, and local rows below off are another CTA's)
+  int row0, m, s0, ns, ng, off = 0;
+  if constexpr (GROUPS) {
+    const GroupRows q = group_rows(H.g, blockIdx.x);
+    s0 = q.s0, ns = q.ns, row0 = 32 * s0, off = q.lo - row0, m = q.hi - row0;
+#pragma unroll 1
+    for (int i = tid; i <= ns; i += kThreads) soff[i] = A.slice_off[s0 + i] - A.slice_off[s0];
+    ng = A.slice_off[s0 + ns] - A.slice_off[s0];
+  } else if (ch == 32) {
     s0 = P.slice0[cta];
     ns = P.slice0[cta + 1] - s0;
     row0 = 32 * s0;
@@ -283,9 +321,9 @@ __global__ void __launch_bounds__(WARPS * 32, 1) pcg_halo_kernel(const __grid_co
     if (tid == 0) soff[0] = 0, soff[1] = ng;
   }
   const int64_t g0 = A.slice_off[s0];  // first block column (chunk 32)
-  const int nh = P.halo_cnt[cta];
+  const int nh = P.halo_cnt[blockIdx.x];
 #pragma unroll 1
-  for (int i = tid; i < nh; i += kThreads) hl[i] = P.halo[(int64_t)cta * P.halo_cap + i];
+  for (int i = tid; i < nh; i += kThreads) hl[i] = P.halo[(int64_t)blockIdx.x * P.halo_cap + i];
   const int per = (ng + WARPS - 1) / WARPS;
   const int ub = min(ng, warp * per), ue = min(ng, ub + per);  // this warp's units
   const int ures = min(ue, ub + resident);                     // [ub, ures) resident, [ures, ue) streamed
@@ -315,7 +353,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1) pcg_halo_kernel(const __grid_co
   // CG state of this lane's components of its rows
   const int rl = STREAM ? lane : lane / 3, comp = STREAM ? 0 : lane - 3 * rl;
   auto row_of = [&](int j) { return (j * WARPS + warp) * kRowsPerWarp + rl; };
-  auto owns = [&](int j) { return (STREAM || lane < 30) && row_of(j) < m; };
+  auto owns = [&](int j) { return (STREAM || lane < 30) && row_of(j) < m && (!GROUPS || row_of(j) >= off); };
   T xr[MAXP][NC], rr[MAXP][NC], zr[MAXP][NC], pr[MAXP][NC], qr[MAXP][NC];
   T mi[kRegM ? MAXP : 1][3 * NC];
   int qfrom[MAXP];  // first partial product of the row (index into qp) and, above bit 20, their number
@@ -328,6 +366,10 @@ __global__ void __launch_bounds__(WARPS * 32, 1) pcg_halo_kernel(const __grid_co
       rr[j][c] = own ? H.r[4 * (int64_t)(row0 + i) + comp + c] : T(0);
       zr[j][c] = pr[j][c] = own ? H.z[4 * (int64_t)(row0 + i) + comp + c] : T(0);
       xr[j][c] = qr[j][c] = T(0);
+      if (GROUPS && own) {
+        pr[j][c] = static_cast<const T*>(H.g.p)[4 * (int64_t)(row0 + i) + comp + c];
+        xr[j][c] = H.x[4 * (int64_t)(row0 + i) + comp + c];
+      }
     }
     if constexpr (kRegM) {
 #pragma unroll
@@ -361,24 +403,35 @@ __global__ void __launch_bounds__(WARPS * 32, 1) pcg_halo_kernel(const __grid_co
       }
     }
   };
-  const double tol2 = H.scal[kTol2];
-  const int maxit = (int)H.scal[kMaxIt];
-  double rrs = H.scal[kRR], rz = H.scal[kRz], beta = 0.0;  // thread 0's
-  int it = (int)H.scal[kIters];
-  int done = (int)H.scal[kDone];
+  double tol2, rrs = 0.0, rz = 0.0, beta = 0.0;  // thread 0's
+  int maxit, it, done, it_end = 0;
+  if constexpr (GROUPS) {
+    const int i = H.g.inst[blockIdx.x];
+    tol2 = H.g.rtol[i] * H.g.rtol[i] * H.g.st[4 * i + 2];
+    maxit = H.g.max_iter;
+    it = H.g.its[i];
+    it_end = it + H.g.chunk;
+    done = 0;
+  } else {
+    tol2 = H.scal[kTol2];
+    maxit = (int)H.scal[kMaxIt];
+    rrs = H.scal[kRR], rz = H.scal[kRz];
+    it = (int)H.scal[kIters];
+    done = (int)H.scal[kDone];
+  }
   if (tid == 0) s_fail = 0;
 
   T* pown = comp == 0 ? px : comp == 1 ? py : pz;  // (a lane per component)
   // the words of sum k for iteration `tag` - 1 in copy c, and one warp forming the CTA's sum from the warps' and
   // writing its word to every copy
   auto sum_words = [&](int k, uint32_t tag, int c) {
-    return H.part + 2 * ((((tag - 1u) & 1u) * kSums + k) * kCopies + c) * kMaxCtas;
+    return part + 2 * ((((tag - 1u) & 1u) * kSums + k) * kCopies + c) * kMaxCtas;
   };
   auto publish_sum = [&](int k, uint32_t tag) {
     // (selects, no branch: a warp that enters the sum diverged takes two thousand cycles for it)
     const int l = lane < nwr ? lane : 0;
     const Num t = warp_sum(lane < nwr ? swS[k][l] >> 4 : 0, lane < nwr ? swx[k][l] : kZeroExp);
-    if (lane < kCopies && !(H.wc.withhold_first && cta == 0 && tag == 1u))
+    if (lane < kCopies && (GROUPS || !(H.wc.withhold_first && cta == 0 && tag == 1u)))
       st_word(sum_words(k, tag, lane) + 2 * cta, (uint64_t)t.S, pack32((uint32_t)t.x, tag));
   };
 
@@ -467,15 +520,29 @@ __global__ void __launch_bounds__(WARPS * 32, 1) pcg_halo_kernel(const __grid_co
       if (!STREAM && ((pend >> j) & 1u)) got[j] = fetch_row(H.p, hl[tid + j * kThreads], tag, vx[j], vy[j], vz[j]);
     }
     if (warp < nwr) {
-      T srz = T(0), srr = T(0);
+      // GROUPS in FP32: r.r as a pair of floats, exact squares and compensated sums (the instances' tolerances go down to
+      // where 24 bits of a lane's squares would show)
+      constexpr bool kPair = GROUPS && sizeof(T) == 4;
+      T srz = T(0), srr = T(0), low = T(0);
 #pragma unroll
       for (int j = 0; j < MAXP; ++j)  // zero where the lane owns nothing
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
           srz += rr[j][c] * zr[j][c];
-          srr += rr[j][c] * rr[j][c];
+          if constexpr (kPair) {
+            const T v = rr[j][c], sq = v * v, t = srr + sq, d = t - srr;
+            low += fma(v, v, -sq) + ((srr - (t - d)) + (sq - d));
+            srr = t;
+          } else {
+            srr += rr[j][c] * rr[j][c];
+          }
         }
-      warp_parts<T>(srz, srr, T(0), &swS[3][warp], &swx[3][warp], WARPS);
+      if constexpr (kPair) {
+        const T t = srr + low;
+        low -= t - srr;
+        srr = t;
+      }
+      warp_parts<T, kPair>(srz, srr, low, &swS[3][warp], &swx[3][warp], WARPS);
     }
 #pragma unroll
     for (int j = 0; j < kBatch; ++j)
@@ -508,7 +575,8 @@ __global__ void __launch_bounds__(WARPS * 32, 1) pcg_halo_kernel(const __grid_co
       T a0 = T(0), a1 = T(0), a2 = T(0);
       auto product = [&](const unsigned char* vals, const unsigned char* cols) {
         const T* v = reinterpret_cast<const T*>(vals) + lane;
-        const int c = reinterpret_cast<const uint16_t*>(cols)[lane];
+        int c = reinterpret_cast<const uint16_t*>(cols)[lane];
+        if (GROUPS) c = min(c, H.np - 1);  // another CTA's row of a shared slice: its column means nothing here
         const T x0 = px[c], x1 = py[c], x2 = pz[c];
         // one multiply-add per entry: as a sum of three products the row would cost a fourth instruction, and nine FP64
         // instructions per block are what bounds the FP64 form
@@ -645,9 +713,9 @@ __global__ void __launch_bounds__(WARPS * 32, 1) pcg_halo_kernel(const __grid_co
         int d = 0;
         double alpha = 0.0;
         // rrs and tol2 are not negative: their order is that of their bits (a NaN is above every number)
-        if (it > 0 && __double_as_longlong(rrs) <= __double_as_longlong(tol2)) d = 1;
-        else if (it > 0 && it >= maxit) d = 2;
-        else if ((__double_as_longlong(pq) << 1) == 0 || ex == 2047) d = 3;  // negative curvature alone does not stop CG
+        if ((GROUPS || it > 0) && __double_as_longlong(rrs) <= __double_as_longlong(tol2)) d = 1;
+        else if ((GROUPS || it > 0) && it >= maxit) d = GROUPS ? 1 : 2;
+        else if ((__double_as_longlong(pq) << 1) == 0 || ex == 2047) d = GROUPS ? 2 : 3;  // negative curvature alone does not stop CG
         else {
           // alpha = rz / pq and beta = (rz - 2 alpha zq + alpha^2 qw) / rz = 1 + (alpha qw - 2 zq) / pq from one
           // reciprocal; sums whose p.q is near the ends of the range are scaled by a power of two
@@ -689,6 +757,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1) pcg_halo_kernel(const __grid_co
       }
     }
     ++it;
+    if (GROUPS && it == it_end) break;
   }
 
   // drain the copies in flight (the cyclic stream runs ahead of the last iteration)
@@ -699,6 +768,36 @@ __global__ void __launch_bounds__(WARPS * 32, 1) pcg_halo_kernel(const __grid_co
       phase ^= 1u << st;
       st = st + 1 == nring ? 0 : st + 1;
     }
+  }
+  if constexpr (GROUPS) {
+    const int inst = H.g.inst[blockIdx.x];
+    if (!failed) {
+#pragma unroll
+      for (int j = 0; j < MAXP; ++j)
+        if (owns(j)) {
+#pragma unroll
+          for (int c = 0; c < NC; ++c) {
+            const int64_t row = row0 + row_of(j), i = 4 * row + comp + c;
+            if (done != 0) {
+              H.g.x_out[3 * row + comp + c] = double(xr[j][c]);
+            } else {  // continued by the next launch
+              H.x[i] = xr[j][c];
+              const_cast<T*>(H.r)[i] = rr[j][c];
+              const_cast<T*>(H.z)[i] = zr[j][c];
+              static_cast<T*>(H.g.p)[i] = pr[j][c];
+            }
+          }
+        }
+    }
+    if (tid == 0 && (cta == 0 || failed)) {
+      if (cta == 0 && !failed) {
+        const double bb = H.g.st[4 * inst + 2];
+        H.g.its[inst] = it;
+        H.g.relres[inst] = bb > 0.0 ? sqrt(rrs / bb) : 0.0;
+      }
+      atomicMin(&H.g.flag[inst], failed ? -1 : done);  // set above every flag before the launch
+    }
+    return;
   }
 #pragma unroll
   for (int j = 0; j < MAXP; ++j)
@@ -721,17 +820,23 @@ __global__ void __launch_bounds__(WARPS * 32, 1) pcg_halo_kernel(const __grid_co
 // ---- the pattern's plan: halo rows and 16-bit local columns, one CTA per CG CTA ---------------------------------
 // own row r is local r - row0; a row outside is m + its rank among the CTA's halo rows (ascending): a bitmap of the
 // referenced rows and the running count of its words give the rank
-__global__ void __launch_bounds__(1024) halo_plan_kernel(Bsr A, HaloPlan P, int32_t* slice0, int32_t* cnt,
+// (GROUPS: per CTA of an instance's group, among the instance's rows; a block of another CTA's row is left alone)
+template <bool GROUPS>
+__global__ void __launch_bounds__(1024) halo_plan_kernel(Bsr A, HaloPlan P, HaloGroups g, int32_t* slice0, int32_t* cnt,
                                                          int32_t* halo, uint16_t* col16) {
   extern __shared__ uint32_t sm[];
   __shared__ int wtot[32];
   __shared__ int carry;
   const int tid = threadIdx.x, cta = blockIdx.x, ch = P.chunk;
-  const int words = (A.n_rows + 31) / 32;
+  const int r0 = GROUPS ? g.node_off[g.inst[cta]] : 0, r1 = GROUPS ? g.node_off[g.inst[cta] + 1] : A.n_rows;
+  const int words = (r1 - r0 + 31) / 32;
   uint32_t* bits = sm;
   int* rank = reinterpret_cast<int*>(sm + words);
-  int row0, m;
-  if (ch == 32) {
+  int row0, m, off = 0;  // local rows [off, m)
+  if constexpr (GROUPS) {
+    const GroupRows q = group_rows(g, cta);
+    row0 = 32 * q.s0, off = q.lo - row0, m = q.hi - row0;
+  } else if (ch == 32) {
     const int sa = (int)((int64_t)cta * A.n_slices / P.n_cta), sb = (int)((int64_t)(cta + 1) * A.n_slices / P.n_cta);
     row0 = 32 * sa;
     m = min(32 * (sb - sa), A.n_rows - row0);
@@ -744,11 +849,11 @@ __global__ void __launch_bounds__(1024) halo_plan_kernel(Bsr A, HaloPlan P, int3
   for (int i = tid; i < words; i += blockDim.x) bits[i] = 0u;
   if (tid == 0) carry = 0;
   __syncthreads();
-  for (int i = tid; i < m; i += blockDim.x) {
+  for (int i = off + tid; i < m; i += blockDim.x) {
     const int row = row0 + i;
     for (int k = A.row_ptr[row]; k < A.row_ptr[row + 1]; ++k) {
-      const int c = A.col[k];
-      if (c < row0 || c >= row0 + m) atomicOr(&bits[c >> 5], 1u << (c & 31));
+      const int c = A.col[k], d = c - r0;
+      if (c < row0 + off || c >= row0 + m) atomicOr(&bits[d >> 5], 1u << (d & 31));
     }
   }
   __syncthreads();
@@ -773,20 +878,48 @@ __global__ void __launch_bounds__(1024) halo_plan_kernel(Bsr A, HaloPlan P, int3
   if (carry > P.halo_cap) return;  // the host sees the count and does not use the plan
   for (int i = tid; i < words; i += blockDim.x) {
     int k = rank[i];
-    for (uint32_t b = bits[i]; b; b &= b - 1) halo[(int64_t)cta * P.halo_cap + k++] = 32 * i + __ffs(b) - 1;
+    for (uint32_t b = bits[i]; b; b &= b - 1) halo[(int64_t)cta * P.halo_cap + k++] = r0 + 32 * i + __ffs(b) - 1;
   }
-  const int mp = ch == 32 ? (m + 31) / 32 * 32 : m;  // lanes without a row get the column 0
-  for (int i = tid; i < mp; i += blockDim.x) {
+  const int mp = !GROUPS && ch == 32 ? (m + 31) / 32 * 32 : m;  // lanes without a row get the column 0
+  for (int i = off + tid; i < mp; i += blockDim.x) {
     const int row = row0 + i, s = row >> 5;
     for (int g = A.slice_off[s]; g < A.slice_off[s + 1]; ++g) {
       const int64_t b = (int64_t)g * 32 + (row & 31);
       int l = 0;
       if (row < A.n_rows) {
-        const int c = A.col_sell[b];
-        l = c >= row0 && c < row0 + m ? c - row0 : m + rank[c >> 5] + __popc(bits[c >> 5] & ((1u << (c & 31)) - 1u));
+        const int c = A.col_sell[b], d = c - r0;
+        l = c >= row0 + off && c < row0 + m ? c - row0 : m + rank[d >> 5] + __popc(bits[d >> 5] & ((1u << (d & 31)) - 1u));
       }
       col16[b] = (uint16_t)l;
     }
+  }
+}
+
+// GROUPS: start of a solve on b.  One CTA per instance: x = 0, r = b, z = M^-1 r, p = z, no published rows, b.b.
+template <typename T>
+__global__ void __launch_bounds__(512) halo_groups_init_kernel(HaloGroups g, const double* __restrict__ b,
+                                                               const T* __restrict__ minv, T* x, T* r, T* z, T* published) {
+  __shared__ double sh[512];
+  if (g.first[blockIdx.x] != (int)blockIdx.x) return;
+  const int inst = g.inst[blockIdx.x];
+  double bb[1] = {0.0};
+  for (int64_t i = g.node_off[inst] + threadIdx.x; i < g.node_off[inst + 1]; i += blockDim.x) {
+    const T v[3] = {T(b[3 * i]), T(b[3 * i + 1]), T(b[3 * i + 2])};
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const T* q = minv + 9 * i + 3 * c;
+      x[4 * i + c] = T(0);
+      r[4 * i + c] = v[c];
+      z[4 * i + c] = static_cast<T*>(g.p)[4 * i + c] = q[0] * v[0] + q[1] * v[1] + q[2] * v[2];
+      bb[0] += double(v[c]) * double(v[c]);
+    }
+#pragma unroll
+    for (int c = 0; c < 4; ++c) published[4 * i + c] = T(0);
+  }
+  cta_reduce_smem<1>(bb, sh);
+  if (threadIdx.x == 0) {
+    g.st[4 * inst + 2] = bb[0];
+    g.its[inst] = 0;
   }
 }
 
@@ -828,9 +961,10 @@ Layout layout_of(const HaloPlan& P, int warps) {
   return L;
 }
 
-template <typename T, int WARPS, int MAXP, int CB>
-cudaError_t launch_variant(const Bsr& A, PcgWork& w, const Layout& L, cudaStream_t s) {
-  auto kern = pcg_halo_kernel<T, WARPS, MAXP, CB>;
+template <typename T, int WARPS, int MAXP, int CB, bool GROUPS = false>
+cudaError_t launch_variant(const Bsr& A, PcgWork& w, const Layout& L, cudaStream_t s, const HaloPlan& P,
+                           const HaloGroups& g = HaloGroups{}) {
+  auto kern = pcg_halo_kernel<T, WARPS, MAXP, CB, GROUPS>;
   static std::mutex mu;
   static bool set[64] = {false};
   int dev = 0;
@@ -844,7 +978,8 @@ cudaError_t launch_variant(const Bsr& A, PcgWork& w, const Layout& L, cudaStream
     }
   }
   HaloArgs<T> H;
-  H.P = *w.halo;
+  H.P = P;
+  H.g = g;
   H.A = A;
   H.val = (const T*)A.val;
   H.minv = (const T*)w.minv;
@@ -871,22 +1006,35 @@ cudaError_t launch(const Bsr& A, PcgWork& w, int variant, cudaStream_t s) {
     const Layout L = layout_of<float>(*w.halo, warps_of(true, variant));
     if (!L.ok) return cudaErrorInvalidConfiguration;
     if (variant == 1)
-      return L.passes <= 1 ? launch_variant<float, 8, 1, 0>(A, w, L, s) : launch_variant<float, 8, 2, 0>(A, w, L, s);
-    if (!L.ring) return L.passes <= 1 ? launch_variant<float, 16, 1, 0>(A, w, L, s) : launch_variant<float, 16, 2, 0>(A, w, L, s);
-    if (L.units == 2) return launch_variant<float, 16, 4, 2>(A, w, L, s);
-    return L.passes <= 1 ? launch_variant<float, 16, 1, 4>(A, w, L, s) : launch_variant<float, 16, 2, 4>(A, w, L, s);
+      return L.passes <= 1 ? launch_variant<float, 8, 1, 0>(A, w, L, s, *w.halo) : launch_variant<float, 8, 2, 0>(A, w, L, s, *w.halo);
+    if (!L.ring) return L.passes <= 1 ? launch_variant<float, 16, 1, 0>(A, w, L, s, *w.halo) : launch_variant<float, 16, 2, 0>(A, w, L, s, *w.halo);
+    if (L.units == 2) return launch_variant<float, 16, 4, 2>(A, w, L, s, *w.halo);
+    return L.passes <= 1 ? launch_variant<float, 16, 1, 4>(A, w, L, s, *w.halo) : launch_variant<float, 16, 2, 4>(A, w, L, s, *w.halo);
   }
   const Layout L = layout_of<double>(*w.halo, warps_of(false, variant));
   if (!L.ok) return cudaErrorInvalidConfiguration;
   if (variant == 1) {
-    if (!L.ring) return launch_variant<double, 16, 2, 0>(A, w, L, s);
-    if (L.units == 1) return launch_variant<double, 16, 2, 1>(A, w, L, s);
-    return L.passes <= 1 ? launch_variant<double, 16, 1, 2>(A, w, L, s) : launch_variant<double, 16, 2, 2>(A, w, L, s);
+    if (!L.ring) return launch_variant<double, 16, 2, 0>(A, w, L, s, *w.halo);
+    if (L.units == 1) return launch_variant<double, 16, 2, 1>(A, w, L, s, *w.halo);
+    return L.passes <= 1 ? launch_variant<double, 16, 1, 2>(A, w, L, s, *w.halo) : launch_variant<double, 16, 2, 2>(A, w, L, s, *w.halo);
   }
-  if (!L.ring) return L.passes <= 1 ? launch_variant<double, 8, 1, 0>(A, w, L, s) : launch_variant<double, 8, 2, 0>(A, w, L, s);
-  if (L.units == 1) return launch_variant<double, 8, 4, 1>(A, w, L, s);
-  if (L.passes <= 1) return launch_variant<double, 8, 1, 2>(A, w, L, s);
-  return L.passes <= 2 ? launch_variant<double, 8, 2, 2>(A, w, L, s) : launch_variant<double, 8, 4, 2>(A, w, L, s);
+  if (!L.ring) return L.passes <= 1 ? launch_variant<double, 8, 1, 0>(A, w, L, s, *w.halo) : launch_variant<double, 8, 2, 0>(A, w, L, s, *w.halo);
+  if (L.units == 1) return launch_variant<double, 8, 4, 1>(A, w, L, s, *w.halo);
+  if (L.passes <= 1) return launch_variant<double, 8, 1, 2>(A, w, L, s, *w.halo);
+  return L.passes <= 2 ? launch_variant<double, 8, 2, 2>(A, w, L, s, *w.halo) : launch_variant<double, 8, 4, 2>(A, w, L, s, *w.halo);
+}
+// The GROUPS form is built with the warps of variant 0.
+template <typename T, int WARPS>
+cudaError_t launch_groups(const Bsr& A, PcgWork& w, const Layout& L, cudaStream_t s, const HaloPlan& P,
+                          const HaloGroups& g) {
+  constexpr int U = sizeof(T) == 8 ? 2 : 4;
+  if (!L.ring)
+    return L.passes <= 1 ? launch_variant<T, WARPS, 1, 0, true>(A, w, L, s, P, g)
+                         : launch_variant<T, WARPS, 2, 0, true>(A, w, L, s, P, g);
+  if (L.units < U) return launch_variant<T, WARPS, 4, U / 2, true>(A, w, L, s, P, g);
+  if (L.passes <= 1) return launch_variant<T, WARPS, 1, U, true>(A, w, L, s, P, g);
+  if (L.passes <= 2) return launch_variant<T, WARPS, 2, U, true>(A, w, L, s, P, g);
+  return launch_variant<T, WARPS, 4, U / (sizeof(T) == 4 ? 2 : 1), true>(A, w, L, s, P, g);
 }
 // variant 1 exists where it can be faster: FP32 without a stream, FP64 up to two passes
 Layout usable(const PcgWork& w, int variant) {
@@ -916,9 +1064,9 @@ int halo_max_rows() { return kSmemBudget / 8 * 32; }
 cudaError_t launch_halo_plan(const Bsr& A, const HaloPlan& P, int32_t* slice0, int32_t* cnt, int32_t* halo,
                              uint16_t* col16, cudaStream_t s) {
   const int bytes = (A.n_rows + 31) / 32 * 8;
-  cudaError_t e = cudaFuncSetAttribute(halo_plan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBudget);
+  cudaError_t e = cudaFuncSetAttribute(halo_plan_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBudget);
   if (e != cudaSuccess) return e;
-  halo_plan_kernel<<<P.n_cta, 1024, bytes, s>>>(A, P, slice0, cnt, halo, col16);
+  halo_plan_kernel<false><<<P.n_cta, 1024, bytes, s>>>(A, P, HaloGroups{}, slice0, cnt, halo, col16);
   return cudaGetLastError();
 }
 
@@ -932,6 +1080,36 @@ bool pcg_halo_eligible(const PcgWork& w, int variant) {
 bool pcg_halo_streams(const PcgWork& w, int variant) { return usable(w, variant).ring > 0; }
 
 static_assert(kHaloWords == 2 * kSums * kCopies * kMaxCtas * 2, "the words' share of the work array");
+
+bool batched_halo_fits(const HaloPlan& P, bool fp32) {
+  return (fp32 ? layout_of<float>(P, warps_of(true, 0)) : layout_of<double>(P, warps_of(false, 0))).ok;
+}
+cudaError_t launch_batched_halo(const Bsr& A, const PcgWork& work, const HaloPlan& P, int32_t* cnt, int32_t* halo,
+                                uint16_t* col16, int max_rows, const double* b, double* x_out, const int32_t* node_off,
+                                const int32_t* cta_inst, const int32_t* cta_first, const int32_t* cta_size,
+                                const double* rtol, int max_iter, int chunk, bool first_launch, double* st, int32_t* its,
+                                int32_t* flag, int n_inst, double* relres, cudaStream_t s) {
+  const Layout L = work.fp32 ? layout_of<float>(P, warps_of(true, 0)) : layout_of<double>(P, warps_of(false, 0));
+  if (!L.ok) return cudaErrorInvalidConfiguration;
+  PcgWork w = work;
+  // the streamed blocks stay in L2 as far as 90 of its 129 MB go
+  const int64_t groups = A.n_padded / 32, kept = (90ll << 20) / (w.fp32 ? unit_bytes<float>() : unit_bytes<double>());
+  w.keep_g = groups < kept ? groups : kept;
+  const HaloGroups g{cta_inst, cta_first, cta_size, node_off, rtol, max_iter, chunk, w.p0, st, its, flag, relres, x_out};
+  cudaError_t e = cudaMemsetAsync(w.part_c, 0, sizeof(double) * kHaloWords, s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(flag, 0x7f, sizeof(int32_t) * n_inst, s);
+  if (e != cudaSuccess) return e;
+  halo_plan_kernel<true><<<P.n_cta, 1024, (max_rows + 31) / 32 * 8, s>>>(A, P, g, nullptr, cnt, halo, col16);
+  if (first_launch && w.fp32)
+    halo_groups_init_kernel<float><<<P.n_cta, 512, 0, s>>>(g, b, (const float*)w.minv, (float*)w.x, (float*)w.r,
+                                                          (float*)w.z, (float*)w.p1);
+  else if (first_launch)
+    halo_groups_init_kernel<double><<<P.n_cta, 512, 0, s>>>(g, b, (const double*)w.minv, (double*)w.x, (double*)w.r,
+                                                           (double*)w.z, (double*)w.p1);
+  e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  return w.fp32 ? launch_groups<float, 16>(A, w, L, s, P, g) : launch_groups<double, 8>(A, w, L, s, P, g);
+}
 
 cudaError_t launch_pcg_halo(const Bsr& A, PcgWork& w, int variant, cudaStream_t s) {
   return usable(w, variant).ok ? launch(A, w, variant, s) : cudaErrorInvalidConfiguration;

@@ -1364,6 +1364,11 @@ struct ikr_nr_s {
     int cur_variant = 0;         // kernels.h launch_batched_pcg variant of the current plan (4: clusters)
     bool cooperative = false;
     DBuf<int32_t> cta_inst, cta_first, cta_size;
+    // one-reduction form (cg_halo.cu): the current split and its lists
+    ikr::HaloPlan halo_split;
+    DBuf<int32_t> halo_cnt, halo_rows;
+    DBuf<uint16_t> col16;
+    int max_rows = 0;            // of the running instances
     DBuf<double> part;
     DBuf<unsigned int> counters;
     DBuf<double> st;             // rz, r.r, b.b, beta per instance between the launches of one solve
