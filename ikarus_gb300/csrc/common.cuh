@@ -44,6 +44,36 @@ struct GpFactors {
     return (v >> d) & 1 ? x : -x;
   }
 };
+// The trilinear interpolation as butterflies over the eight lanes of an element: lane v holds the value at node v and gets
+// that at Gauss point v, bit d of both being the side in direction d.  Along a direction the interpolation is
+// own + Lo (other - own) and the derivative the difference of the two sides, so the three derivatives of a field take 12
+// FP64 instructions instead of the 24 of a sum over the nodes, and the transposed operation 15 instead of 24 and the sum
+// over the points.  All 32 lanes take part.
+struct GpButterfly {
+  uint32_t sign[3];  // the sign bit, set on the high side of a direction
+  __device__ __forceinline__ explicit GpButterfly(int q) {
+#pragma unroll
+    for (int d = 0; d < 3; ++d) sign[d] = (uint32_t)((q >> d) & 1) << 31;
+  }
+  static __device__ __forceinline__ double other(double x, int d) { return __shfl_xor_sync(0xffffffffu, x, 1 << d); }
+  static __device__ __forceinline__ double flip(double x, uint32_t s) {
+    return __hiloint2double((int)((uint32_t)__double2hiint(x) ^ s), __double2loint(x));
+  }
+  static __device__ __forceinline__ double along(double x, int d) { return fma(kGaussLo, other(x, d) - x, x); }
+  __device__ __forceinline__ void gradient(double u, double (&g)[3]) const {
+    const double dz = other(u, 2) - u, t = fma(kGaussLo, dz, u);
+    g[0] = along(flip(other(t, 0) - t, sign[0]), 1);
+    g[1] = along(flip(other(t, 1) - t, sign[1]), 0);
+    g[2] = along(along(flip(dz, sign[2]), 1), 0);
+  }
+  // sum over the points of q . dN_v/dxi
+  __device__ __forceinline__ double onto_nodes(const double (&q)[3]) const {
+    double s[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) s[d] = flip(q[d] + other(q[d], d), sign[d] ^ 0x80000000u);
+    return along(along(s[0], 1) + along(s[1], 0), 2) + along(along(s[2], 1), 0);
+  }
+};
 // dN_v/dxi at the element centre (1/2,1/2,1/2)
 template <typename T>
 __device__ __forceinline__ void ref_gradient_at_center(int v, T dxi[3]) {

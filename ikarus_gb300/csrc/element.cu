@@ -599,16 +599,15 @@ __global__ void traction_kernel(const double* __restrict__ X, const int32_t* __r
 }
 
 // FP64 element forces (24 per listed element) with the material work spread over the Gauss points: lane q of an element's 8 lanes
-// evaluates Gauss point q (geometry J, dN/dX of all 8 nodes, F, F^-1, ln J, P) once, instead of every lane
-// evaluating every Gauss point; the nodal forces w P dN_v of each point are exchanged through shared memory and
-// lane v sums its node's over the points in ascending order.  About a quarter of the FP64 operations of the
-// node-per-lane form, which matters because GB300's FP64 rate bounds this kernel: about 480 FP64 instructions per lane.
-// Measured with the gather: 131 072 elements 0.97 ms (eight coloured launches) -> 0.83 ms, 256 elements 165 -> 21 us.
+// evaluates Gauss point q (geometry J, F, F^-1, ln J, P) once, instead of every lane evaluating every Gauss point.
+// What bounds it is GB300's FP64 rate, so the interpolation of X and u and the sum of the nodal forces over the points run as
+// butterflies over the eight lanes (GpButterfly): about 340 FP64 instructions per lane, 480 with sums over nodes and
+// points, a quarter of the node-per-lane form.
+// Measured: 131 072 elements 0.82 -> 0.60 ms (node-per-lane lists in eight coloured launches 0.97), 256 elements 165 -> 20 us.
 // HYP: the hyperelastic framework's material point (a separate instantiation keeps the other laws' registers)
 template <int EPB, bool HYP>
 __global__ void __launch_bounds__(EPB * 8) disp_residual_gp_kernel(ElemArgs a, const int32_t* __restrict__ list,
                                                                     int n_list, int e_base) {
-  __shared__ double fs[EPB][8][8][3];  // [element][Gauss point][node][component]
   const int lane = threadIdx.x & 31;
   const int sub = threadIdx.x & 7;  // node for loads and the scatter, Gauss point for the material work
   const int es = threadIdx.x >> 3;
@@ -633,20 +632,13 @@ __global__ void __launch_bounds__(EPB * 8) disp_residual_gp_kernel(ElemArgs a, c
     dU[c] = Ud[c] - __shfl_sync(0xffffffffu, Ud[c], src);
   }
   const double lam = a.lam_e ? a.lam_e[e] : a.lam, mu = a.mu_e ? a.mu_e[e] : a.mu;
-  const GpFactors dxi(sub);
-  // J = sum_v dX_v (x) dxi_v and the same of dU; F = I + (sum_v dU_v (x) dxi_v) J^-1
-  double J[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}}, G[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
+  const GpButterfly fly(sub);
+  // J = sum_v dX_v (x) dN_v/dxi and the same of dU; F = I + (sum_v dU_v (x) dN_v/dxi) J^-1
+  double J[3][3], G[3][3];
 #pragma unroll
-  for (int v = 0; v < 8; ++v) {
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-      const double x = __shfl_sync(0xffffffffu, dX[i], src + v), u = __shfl_sync(0xffffffffu, dU[i], src + v);
-#pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        J[i][d] = fma(x, dxi(v, d), J[i][d]);
-        G[i][d] = fma(u, dxi(v, d), G[i][d]);
-      }
-    }
+  for (int i = 0; i < 3; ++i) {
+    fly.gradient(dX[i], J[i]);
+    fly.gradient(dU[i], G[i]);
   }
   double Ji[3][3];
   const double detJ = inv3(J, Ji);
@@ -713,12 +705,12 @@ __global__ void __launch_bounds__(EPB * 8) disp_residual_gp_kernel(ElemArgs a, c
     const double detF = inv3(F, Fi);
     // det C = det(F)^2 must exceed 1e-10 (checkPositiveOrAbort); NaN fails the test as well
     if (!(detF * detF > 1e-10) || !(detF > 0.0)) bad |= kStatusNonPositiveDetC;
-    const double lnJ = log(detF);
     // P = mu (F - F^-T) + lambda ln J F^-T (F - F^-T keeps the undeformed internal force exactly zero)
+    const double wl = w * lam * log(detF), wm = w * mu;
 #pragma unroll
     for (int i = 0; i < 3; ++i)
 #pragma unroll
-      for (int j = 0; j < 3; ++j) P[i][j] = w * (mu * (F[i][j] - Fi[j][i]) + lam * lnJ * Fi[j][i]);
+      for (int j = 0; j < 3; ++j) P[i][j] = wm * (F[i][j] - Fi[j][i]) + wl * Fi[j][i];
   }
   // w P dN_v = (w P J^-T) dxi_v: no gradient is formed
   double Q[3][3];
@@ -726,17 +718,9 @@ __global__ void __launch_bounds__(EPB * 8) disp_residual_gp_kernel(ElemArgs a, c
   for (int i = 0; i < 3; ++i)
 #pragma unroll
     for (int d = 0; d < 3; ++d) Q[i][d] = P[i][0] * Ji[d][0] + P[i][1] * Ji[d][1] + P[i][2] * Ji[d][2];
+  double f[3];
 #pragma unroll
-  for (int v = 0; v < 8; ++v)
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-      fs[es][sub][v][i] = fma(Q[i][0], dxi(v, 0), fma(Q[i][1], dxi(v, 1), Q[i][2] * dxi(v, 2)));
-  __syncwarp();
-  double f[3] = {0.0, 0.0, 0.0};
-#pragma unroll
-  for (int g = 0; g < 8; ++g)
-#pragma unroll
-    for (int i = 0; i < 3; ++i) f[i] += fs[es][g][sub][i];
+  for (int i = 0; i < 3; ++i) f[i] = fly.onto_nodes(Q[i]);
   if (a.trac_idx) {
     const int t = a.trac_idx[e];
     if (t >= 0) {
