@@ -149,53 +149,119 @@ __global__ void __launch_bounds__(256) coarse_prolong_kernel(Coarse C, T* z, con
   }
 }
 
+// Lane sums of the 36 entries in v: halves are exchanged, so the butterfly takes 37 additions instead of 180.  The lane ends
+// with the sums of entries first .. first + n - 1 (n <= 2) in v[0], v[1].
+template <int SIZE, int M>
+__device__ __forceinline__ void reduce_step(double (&v)[36], int lane, int& first, int& n) {
+  constexpr int kHalf = (SIZE + 1) / 2;
+  const bool up = lane & M;
+#pragma unroll
+  for (int k = 0; k < kHalf; ++k) {
+    const double hi = kHalf + k < SIZE ? v[kHalf + k] : 0.0;
+    v[k] = (up ? hi : v[k]) + __shfl_xor_sync(0xffffffffu, up ? v[k] : hi, M);
+  }
+  first += up ? kHalf : 0;
+  n = up ? n - kHalf : min(n, kHalf);
+  if constexpr (M > 1) reduce_step<kHalf, M / 2>(v, lane, first, n);
+}
+__device__ __forceinline__ void reduce_36(double (&v)[36], int lane, int& first, int& n) {
+  first = 0, n = 36;
+  reduce_step<36, 16>(v, lane, first, n);
+}
+
+// float to double of zeros and normal numbers on the integer pipe (a conversion instruction is as slow as the FP64 ones)
+__device__ __forceinline__ bool widens(float f) {
+  const uint32_t m = __float_as_uint(f) & 0x7fffffffu;
+  return m == 0 || m - 0x800000u < 0x7f000000u;
+}
+__device__ __forceinline__ double widened(float f) {
+  const uint32_t b = __float_as_uint(f), m = b & 0x7fffffffu;
+  return __hiloint2double((int)((b & 0x80000000u) | (m ? (m >> 3) + (896u << 20) : 0u)), (int)(b << 29));
+}
+__device__ __forceinline__ bool widens(double) { return true; }
+__device__ __forceinline__ double widened(double v) { return v; }
+
+// part[((d + reach) * n_parts + part) * 36 + 6 r + m], one CTA per run of kGalerkinRows nodes of a chunk: a thread forms
+// W = sum_j K_ij P_j of its row i over the columns of aggregate b + d, the CTA sums P_i^T W.  Bound by the FP64 pipe (27
+// operations per block and, before, twelve conversions), so only the distances that a row of the CTA has are walked, P_i^T W
+// takes its 36 operations and the sums share the butterfly.  140 481 rows of 27 blocks, 16 slabs, FP32: 0.83 -> 0.47 ms (0.66
+// with conversion instructions).  Where nodes are numbered along the slabs' axis, every warp has rows of all three distances
+// and walks 45 blocks instead of 27.
 constexpr int kGalerkinRows = 256;
-// part[((d + reach) * n_parts + part) * 36 + 6 r + m], one CTA per run of kGalerkinRows nodes of a chunk
 template <typename T>
 __global__ void __launch_bounds__(kGalerkinRows) coarse_galerkin_kernel(Coarse C, Bsr A, const T* __restrict__ val,
                                                                         int reach, int runs, double* __restrict__ part) {
   __shared__ double sh[kGalerkinRows / 32][36];
-  const int chunk = blockIdx.x / runs, run = blockIdx.x - chunk * runs;
+  const int chunk = blockIdx.x / runs, run = blockIdx.x - chunk * runs, lane = threadIdx.x & 31;
   const int i = C.chunk_off[chunk] + run * kGalerkinRows + threadIdx.x;
   const bool active = i < C.chunk_off[chunk + 1];
   const int node = active ? __ldg(C.nodes + i) : 0;
   const NodeP n = node_p(C.y4, node);
-  double P[3][6];
-  p_cols(n, P);
   const int g0 = A.slice_off[node >> 5], width = active ? A.slice_off[(node >> 5) + 1] - g0 : 0, l = node & 31;
+  unsigned mine = 0;  // bit d + reach: the row has a column in aggregate b + d
+#pragma unroll 4
+  for (int k = 0; k < width; ++k) {
+    const int J = __ldg(A.col_sell + 32 * (int64_t)(g0 + k) + l);
+    mine |= 1u << (node_p(C.y4, J).agg - n.agg + reach);
+  }
   for (int d = -reach; d <= reach; ++d) {
+    const bool any = (mine >> (d + reach)) & 1u;
+    double* out = part + ((size_t)(d + reach) * gridDim.x + blockIdx.x) * 36;
+    if (!__syncthreads_or(any)) {  // no row of this run couples with aggregate b + d
+      if (threadIdx.x < 36) out[threadIdx.x] = 0.0;
+      continue;
+    }
     double W[3][6] = {};
-    bool any = false;
-    for (int k = 0; k < width; ++k) {
+    for (int k = 0; any && k < width; ++k) {
       const int J = __ldg(A.col_sell + 32 * (int64_t)(g0 + k) + l);
       const NodeP nj = node_p(C.y4, J);
       if (nj.agg != n.agg + d) continue;
-      any = true;
       const T* v = val + (int64_t)(g0 + k) * 288 + l;
-      const double y0 = nj.y[0], y1 = nj.y[1], y2 = nj.y[2];
-      const bool m0 = nj.mask & 1, m1 = nj.mask & 2, m2 = nj.mask & 4;
+      T t[3][3];
+      bool normal = widens(nj.y[0]) && widens(nj.y[1]) && widens(nj.y[2]);
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+          t[c][q] = (nj.mask >> q) & 1 ? __ldg(v + 96 * c + 32 * q) : T(0);
+          normal = normal && widens(t[c][q]);
+        }
+      double y0 = widened(nj.y[0]), y1 = widened(nj.y[1]), y2 = widened(nj.y[2]), a[3][3];
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+#pragma unroll
+        for (int q = 0; q < 3; ++q) a[c][q] = widened(t[c][q]);
+      if (!normal) {
+        asm volatile("");  // a branch: as selects the conversions would run for every block
+        y0 = nj.y[0], y1 = nj.y[1], y2 = nj.y[2];
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+#pragma unroll
+          for (int q = 0; q < 3; ++q) a[c][q] = t[c][q];
+      }
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        const double a0 = m0 ? double(__ldg(v + 96 * c)) : 0.0, a1 = m1 ? double(__ldg(v + 96 * c + 32)) : 0.0,
-                     a2 = m2 ? double(__ldg(v + 96 * c + 64)) : 0.0;
+        const double a0 = a[c][0], a1 = a[c][1], a2 = a[c][2];
         W[c][0] += a0, W[c][1] += a1, W[c][2] += a2;
         W[c][3] = fma(a2, y1, fma(-a1, y2, W[c][3]));  // e_k x y
         W[c][4] = fma(a0, y2, fma(-a2, y0, W[c][4]));
         W[c][5] = fma(a1, y0, fma(-a0, y1, W[c][5]));
       }
     }
-    double* out = part + ((size_t)(d + reach) * gridDim.x + blockIdx.x) * 36;
-    if (!__syncthreads_or(any)) {  // no row of this run couples with aggregate b + d
-      if (threadIdx.x < 36) out[threadIdx.x] = 0.0;
-      continue;
+    double v[36];  // P_i^T W: the free components, and y_i x them
+    const double y0 = n.y[0], y1 = n.y[1], y2 = n.y[2];
+#pragma unroll
+    for (int m = 0; m < 6; ++m) {
+      const double w0 = (n.mask & 1) ? W[0][m] : 0.0, w1 = (n.mask & 2) ? W[1][m] : 0.0, w2 = (n.mask & 4) ? W[2][m] : 0.0;
+      v[m] = w0, v[6 + m] = w1, v[12 + m] = w2;
+      v[18 + m] = fma(y1, w2, -y2 * w1);
+      v[24 + m] = fma(y2, w0, -y0 * w2);
+      v[30 + m] = fma(y0, w1, -y1 * w0);
     }
-#pragma unroll
-    for (int r = 0; r < 6; ++r)
-#pragma unroll
-      for (int m = 0; m < 6; ++m) {
-        const double t = warp_sum(P[0][r] * W[0][m] + P[1][r] * W[1][m] + P[2][r] * W[2][m]);
-        if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5][6 * r + m] = t;
-      }
+    int first, cnt;
+    reduce_36(v, lane, first, cnt);
+    if (cnt > 0) sh[threadIdx.x >> 5][first] = v[0];
+    if (cnt > 1) sh[threadIdx.x >> 5][first + 1] = v[1];
     __syncthreads();
     if (threadIdx.x < 36) {
       double t = 0.0;
