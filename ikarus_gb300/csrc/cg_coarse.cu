@@ -2,9 +2,9 @@
 //
 //   M^-1 r = D^-1 r + P A_c^-1 P^T r          (coarse.cu: the aggregates, P and A_c = P^T K P)
 //
-// The iteration of cg_persistent.cu (product phase with p_new = z + beta p_old formed for every gathered
-// neighbour, grid reduction of p.q, update phase on the owned rows kept in registers) with the coarse part after
-// the update phase, instead of the two extra kernels per iteration of the two-kernel form:
+// The iteration of cg_persistent.cu (product phase, grid reduction of p.q, update phase on the owned rows kept in
+// registers) with the coarse part after the update phase, instead of the two extra kernels per iteration of the two-kernel
+// form:
 //   1. every row adds its six mode sums P_row^T r_row into a per-warp shared array (runs of equal aggregate over
 //      the lanes of a slice are summed by a segmented warp scan, the run totals added in lane order); the CTA adds
 //      its warps' arrays in warp order and publishes, with r.D^-1 r and r.r (FP64), one partial per coarse dof;
@@ -15,8 +15,10 @@
 //      r_c.e.  The mode sums (rows, warps, CTAs), their warp scan and this product run in the CG's type (FP32 for
 //      the FP32 CG: GB300's FP64 pipe is a small fraction of its FP32 rate, and e is kept in the CG's type
 //      anyway); r.D^-1 r, r.r and r_c.e are FP64;
-//   4. the owned rows' z = D^-1 r + P e goes to registers and to the global z the gathers read; a third grid
-//      barrier (arrive and wait) publishes it before the next product phase.
+//   4. the owned rows' z = D^-1 r + P e and p = z + beta p stay in registers, p also goes to the global vector the
+//      gathers read; a third grid barrier (arrive and wait) publishes it before the next product phase.  beta is known
+//      before that barrier, so a neighbour costs one gather, where p formed from z and the old p per neighbour took two:
+//      at 140 481 rows, 16 slabs, FP32 40.9 -> 36.6 us per iteration.
 // Before the first iteration the same coarse part turns the init kernel's z = D^-1 r_0 into M^-1 r_0.  All sums
 // have a fixed order: a solve is bit-identical run to run.  Every wait is bounded (grid barriers and stage waits
 // give up with scal[kDone] = 6 after their poll limits).
@@ -70,8 +72,8 @@ __device__ __forceinline__ bool grid_sync(unsigned int* count, unsigned int targ
 
 template <typename T, int CB, int NST, int WARPS, int MAXS>
 __global__ void __launch_bounds__(WARPS * 32, 1)
-    pcg_coarse_kernel(Bsr A, const T* __restrict__ val, const T* __restrict__ minv, T* x, const T* r, T* z, T* p0,
-                      T* p1, double* scal, Coarse Cc, double* part_a, double* cpart, int64_t keep_g, WaitCtl wc,
+    pcg_coarse_kernel(Bsr A, const T* __restrict__ val, const T* __restrict__ minv, T* x, const T* r, const T* z, T* p,
+                      double* scal, Coarse Cc, double* part_a, double* cpart, int64_t keep_g, WaitCtl wc,
                       int ainv_shared) {
   using C = PersistentCfg<T, CB, NST, WARPS>;
   extern __shared__ __align__(128) unsigned char smem[];
@@ -130,7 +132,6 @@ __global__ void __launch_bounds__(WARPS * 32, 1)
   // FP64 scalars: rz, r.r and beta are thread 0's (the others' copies are not updated); every thread keeps the
   // stop decision, the iteration count and beta in the CG's type
   double rz = 0.0, rrs = scal[kRR], done = scal[kDone], beta = 0.0;
-  T tbv = T(0);
   int it = (int)scal[kIters];
 
   if (ainv_shared) {
@@ -147,8 +148,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1)
   unsigned int barrier_no = 0;
   int loop = 0;
 
-  // The coarse part of z = M^-1 r for the owned rows (zr holds D^-1 r on entry, z = M^-1 r on return, also stored
-  // to the global z): returns false when a grid wait gave up.  Sets rzs (r.z), rrn (r.r).
+  // The coarse part of z = M^-1 r for the owned rows (zr holds D^-1 r on entry, z = M^-1 r on return): returns false when a grid wait gave up.  Sets rzs (r.z), rrn (r.r).
   auto coarse_part = [&](double& rzs, double& rrn) -> bool {
     for (int i = threadIdx.x; i < WARPS * nc; i += blockDim.x) accw[i] = T(0);
     __syncthreads();
@@ -313,9 +313,18 @@ __global__ void __launch_bounds__(WARPS * 32, 1)
       if (!(yp[j].mask & 2)) d1 = T(0);
       if (!(yp[j].mask & 4)) d2 = T(0);
       zr[j][0] += d0, zr[j][1] += d1, zr[j][2] += d2;
-      store3(z, 32 * (gw + j * nw) + lane, zr[j][0], zr[j][1], zr[j][2]);
     }
     return true;
+  };
+  // p = z + tb p on the owned rows; every CTA has read the last p (the reduction of p.q came after its product phase)
+  auto publish_p = [&](T tb) {
+#pragma unroll
+    for (int j = 0; j < MAXS; ++j) {
+      if (yp[j].agg < 0) continue;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) pr[j][c] = zr[j][c] + tb * pr[j][c];
+      store3(p, 32 * (gw + j * nw) + lane, pr[j][0], pr[j][1], pr[j][2]);
+    }
   };
 
   auto issue = [&](int st, const CyclicPos& P) {
@@ -349,6 +358,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1)
     // z_0 = M^-1 r_0 and r_0.z_0
     double rr0 = 0.0;
     if (!coarse_part(rz, rr0)) failed = true;
+    else publish_p(T(0));
     ++barrier_no;
     if (!failed && !grid_sync(bar_count, barrier_no * (unsigned)G, &ok_sh, wc.polls)) failed = true;
     ++loop;
@@ -362,9 +372,6 @@ __global__ void __launch_bounds__(WARPS * 32, 1)
   }
 
   while (done == 0.0 && !failed) {
-    const T tb = tbv;
-    const T* pold = (it & 1) ? p0 : p1;
-    T* pnew = (it & 1) ? p1 : p0;
     T pql = T(0);  // a lane's p.q in the CG's type, converted once
     // ---- product phase: q = K p_new over the owned slices
 #pragma unroll
@@ -385,16 +392,13 @@ __global__ void __launch_bounds__(WARPS * 32, 1)
           int cols[CB];
 #pragma unroll
           for (int k = 0; k < CB; ++k) cols[k] = k < nb ? scol[32 * k + lane] : 0;
-          V3<T> zc[CB], pc[CB];
+          V3<T> pc[CB];
 #pragma unroll
-          for (int k = 0; k < CB; ++k) {
-            zc[k] = load3rw(z, cols[k]);
-            pc[k] = load3rw(pold, cols[k]);
-          }
+          for (int k = 0; k < CB; ++k) pc[k] = load3rw(p, cols[k]);
 #pragma unroll
           for (int k = 0; k < CB; ++k) {
             if (k < nb) {
-              const T x0 = zc[k].x + tb * pc[k].x, x1 = zc[k].y + tb * pc[k].y, x2 = zc[k].z + tb * pc[k].z;
+              const T x0 = pc[k].x, x1 = pc[k].y, x2 = pc[k].z;
               const T* v = sval + 288 * k + lane;
               acc3[0] += v[0] * x0 + v[32] * x1 + v[64] * x2;
               acc3[1] += v[96] * x0 + v[128] * x1 + v[160] * x2;
@@ -408,13 +412,8 @@ __global__ void __launch_bounds__(WARPS * 32, 1)
           st = (st + 1 == NST) ? 0 : st + 1;
         }
         const int row = 32 * (gw + j * nw) + lane;
-        const T n0 = zr[j][0] + tb * pr[j][0], n1 = zr[j][1] + tb * pr[j][1], n2 = zr[j][2] + tb * pr[j][2];
-        pr[j][0] = n0, pr[j][1] = n1, pr[j][2] = n2;
         qr[j][0] = acc3[0], qr[j][1] = acc3[1], qr[j][2] = acc3[2];
-        if (row < A.n_rows) {
-          store3(pnew, row, n0, n1, n2);
-          pql += n0 * acc3[0] + n1 * acc3[1] + n2 * acc3[2];
-        }
+        if (row < A.n_rows) pql += pr[j][0] * acc3[0] + pr[j][1] * acc3[1] + pr[j][2] * acc3[2];
       }
     }
     // ---- grid reduction of p.q
@@ -455,7 +454,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1)
           zr[j][b] = __ldg(m + 3 * b) * rr_[j][0] + __ldg(m + 3 * b + 1) * rr_[j][1] + __ldg(m + 3 * b + 2) * rr_[j][2];
       }
     }
-    // ---- coarse part, r.z, r.r (one grid barrier inside), then publish z (a second)
+    // ---- coarse part, r.z, r.r (one grid barrier inside), then publish p (a second)
     double rzs = 0.0;
     if (!coarse_part(rzs, rrs)) {
       failed = true;
@@ -470,12 +469,12 @@ __global__ void __launch_bounds__(WARPS * 32, 1)
     }
     __syncthreads();
     ++it;
-    tbv = s_tb;
     ++loop;
     if (s_state != 0) {  // every CTA decides alike (the same sums)
       done = s_state;
       break;
     }
+    publish_p(s_tb);
     ++barrier_no;
     if (!grid_sync(bar_count, barrier_no * (unsigned)G, &ok_sh, wc.polls)) {
       failed = true;
@@ -545,9 +544,8 @@ cudaError_t launch_coarse_cfg(const Bsr& A, PcgWork& w, const Coarse& Cc, cudaSt
   const T* minv = (const T*)w.minv;
   T* x = (T*)w.x;
   const T* r = (const T*)w.r;
-  T* z = (T*)w.z;
-  T* p0 = (T*)w.p0;
-  T* p1 = (T*)w.p1;
+  const T* z = (const T*)w.z;
+  T* p = (T*)w.p0;
   double* scal = w.scal;
   Bsr Acopy = A;
   Coarse Ccopy = Cc;
@@ -556,7 +554,7 @@ cudaError_t launch_coarse_cfg(const Bsr& A, PcgWork& w, const Coarse& Cc, cudaSt
   int64_t keep = w.keep_g;
   WaitCtl wc{w.barrier_polls > 0 ? w.barrier_polls : kBarrierSpinLimit, 0};
   int ash = ainv_shared;
-  void* args[] = {&Acopy, &val, &minv, &x, &r, &z, &p0, &p1, &scal, &Ccopy, &pa, &cp, &keep, &wc, &ash};
+  void* args[] = {&Acopy, &val, &minv, &x, &r, &z, &p, &scal, &Ccopy, &pa, &cp, &keep, &wc, &ash};
   return cudaLaunchCooperativeKernel((const void*)kern, dim3(grid), dim3(C::kThreads), args, smem, s);
 }
 
