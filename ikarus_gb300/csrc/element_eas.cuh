@@ -6,14 +6,16 @@
 // and the ansatz spaces easvariants/{linearandglstrains,displacementgradient,helperfunctions}.hh.
 //
 // One element per block of 64 threads: eight lanes (lane = node I) for each of the eight Gauss points, because the work
-// at a point is about 1 800 dependent FP64 instructions a lane, which GB300 starts one per 16 cycles and SM and finishes
+// at a point is some 800 to 1 300 FP64 instructions a lane, many of them dependent, which GB300 starts one per 16 cycles and SM and finishes
 // one per 60: an element whose points follow one another keeps a small mesh waiting for eight times that, and one lane
-// factorising D keeps the other seven.  Measured against eight lanes per element and one launch per colour, residual and
-// tangent with assembly: 10 elements 660 -> 60 us and 1 030 -> 80 us, 8 192 elements 2.34 -> 1.01 ms and 3.86 -> 1.63 ms.
+// factorising D keeps the other seven.  The loops over modes, columns and blocks are rolled: unrolled, the kernels had 120 to
+// 280 KB of instructions, each run once, and now have 70 to 120.  Measured with assembly, residual and tangent, eight
+// lanes per element and one launch per colour -> unrolled -> this: 10 elements (H9) 660 -> 60 -> 46 us and 1 030 -> 80 -> 67 us,
+// 8 192 elements (E9) 2.34 -> 1.01 -> 0.75 ms and 3.86 -> 1.63 -> 1.35 ms.
 // The lanes of a point share F, S and the Voigt tangent C (each lane computes a few of its 36 entries into shared
 // memory), and each lane computes the enhanced-strain columns E_alpha(:,k) and C E_alpha(:,k) for k = I, I+8, ...
-// The points' shares of f, K, L, D and R~ are summed in point order through shared memory.  D (n_alpha x n_alpha) is
-// LU-factorised with a lane per row (partial pivoting, FP64), the 24 columns of D^{-1} L and D^{-1} R~ are solved with
+// The points' shares of f, K, L, D and R~ are summed in a fixed order through shared memory.  D (n_alpha x n_alpha) is
+// LU-factorised by a warp (partial pivoting, FP64), the 24 columns of D^{-1} L and D^{-1} R~ are solved with
 // a lane each, and the condensed quantities
 //   f_I -= L_I^T D^{-1} R~,   K_IJ -= L_I^T D^{-1} L_J        (enhancedassumedstrains.hh:291-296, 336-345)
 // are formed by all 64 threads; K as the 40 blocks (I, I + d mod 8), d = 0..4, d = 1..3 transposed as well.
@@ -46,24 +48,24 @@ __constant__ int kF2[21] = {-1, -1, -1, -1, -1, -1, -1, -1, -1, 1, 2, 1, 2, 2, 2
 template <int NA>
 struct EasCfg {
   static constexpr int NT = NA * (NA + 1) / 2; // packed upper triangle of D
-  static constexpr int DSH = (NT + 7) / 8;     // D entries per lane
-  static constexpr int RSH = (NA + 7) / 8;     // R~ entries per lane
   // shared memory of a Gauss point (doubles)
   static constexpr int O_DN = 0;               // 8 x 3   modified nodal gradients
   static constexpr int O_C6 = O_DN + 24;       // 36      Voigt tangent
   static constexpr int O_EA = O_C6 + 36;       // NA x 6  E_alpha columns
   static constexpr int O_CEA = O_EA + 6 * NA;  // NA x 6  C E_alpha columns
-  static constexpr int POINT = O_CEA + 6 * NA;
+  static constexpr int O_S = O_CEA + 6 * NA;   // NA x 6  GL: ansatz coefficients / detJ times alpha; H/HT: v and coef
+  static constexpr int POINT = O_S + 6 * NA;
   // of the element: the points' shares [share][point], shares in the order f or K, L, D, R~
-  static constexpr int shares(bool want_k) { return (want_k ? 360 : 24) + 24 * NA + NT + NA; }
-  // after the points: T0^{-1} (GL), D, R~ and its solution, L, D^{-1} L, the row order
+  static constexpr int shares(bool want_k) { return (want_k ? 360 : 24) + 24 * NA + NT + (want_k ? 0 : NA); }
+  // after the points: T0^{-1} (GL) or A0 and Fc0 A0 (H/HT), D, R~ and its solution, L, D^{-1} L, the row order
   static constexpr int O_GEO = 8 * POINT;
   static constexpr int O_D = O_GEO + 36;
   static constexpr int O_RT = O_D + NA * NA;
   static constexpr int O_L = O_RT + 2 * NA;    // NA x 24
   static constexpr int O_Y = O_L + 24 * NA;    // 24 x NA
   static constexpr int O_PERM = O_Y + 24 * NA; // NA
-  static constexpr int O_SHARE = O_PERM + NA;
+  static constexpr int O_INV = O_PERM + NA;    // NA      reciprocal pivots
+  static constexpr int O_SHARE = O_INV + NA;
   static constexpr int total(bool want_k) { return O_SHARE + 8 * shares(want_k); }
 };
 
@@ -133,10 +135,6 @@ __global__ void __launch_bounds__(64) eas_element_kernel(ElemArgs a, const int32
     dX[c] = x - __shfl_sync(0xffffffffu, x, src);
     dU[c] = Ud[c] - __shfl_sync(0xffffffffu, Ud[c], src);
   }
-  double al[NA];
-#pragma unroll
-  for (int p = 0; p < NA; ++p) al[p] = a.alpha[(size_t)p * ne + e];
-
   // centre data
   double A0[3][3] = {}, detJ0 = 0.0, dN0[3] = {0, 0, 0}, Fc0[3][3] = {}, Fa[3][3] = {};
   if (KIND == 1) {
@@ -147,6 +145,7 @@ __global__ void __launch_bounds__(64) eas_element_kernel(ElemArgs a, const int32
 #pragma unroll
       for (int j = 0; j < 3; ++j) A0[i][j] = a.eas_geo[(size_t)(3 * i + j) * ne + e];
     detJ0 = a.eas_geo[(size_t)9 * ne + e];
+    if (threadIdx.x < 9) smem[Cfg::O_GEO + threadIdx.x] = a.eas_geo[(size_t)threadIdx.x * ne + e];
     if (KIND == 3) {
 #pragma unroll
       for (int k = 0; k < 3; ++k) dN0[k] = a.eas_geo[(size_t)(10 + 3 * sub + k) * ne + e];
@@ -158,6 +157,12 @@ __global__ void __launch_bounds__(64) eas_element_kernel(ElemArgs a, const int32
       for (int i = 0; i < 3; ++i)
 #pragma unroll
         for (int c = 0; c < 3; ++c) Fa[i][c] = Fc0[i][0] * A0[0][c] + Fc0[i][1] * A0[1][c] + Fc0[i][2] * A0[2][c];
+      if (threadIdx.x == 0) {
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+          for (int c = 0; c < 3; ++c) smem[Cfg::O_GEO + 9 + 3 * i + c] = Fa[i][c];
+      }
     }
   }
   __syncthreads();
@@ -167,7 +172,6 @@ __global__ void __launch_bounds__(64) eas_element_kernel(ElemArgs a, const int32
   double* share = smem + Cfg::O_SHARE + q;  // share t of this point at share[8 t]
   constexpr int kL = WANT_K ? 360 : 24, kD = kL + 24 * NA, kR = kD + Cfg::NT;
   {
-    const double xi[3] = {(q & 1) ? kGaussHi : kGaussLo, (q & 2) ? kGaussHi : kGaussLo, (q & 4) ? kGaussHi : kGaussLo};
     double dxi[3];
     ref_gradient_at_gp<double>(sub, q, dxi);
     double J[3][3];
@@ -187,28 +191,38 @@ __global__ void __launch_bounds__(64) eas_element_kernel(ElemArgs a, const int32
       for (int j = 0; j < 3; ++j) H[i][j] = sum8(dU[i] * dN[j]);
 
     // enhancement at this Gauss point
-    double s[NA];  // H/HT mode scales, GL ansatz coefficients / detJ
+    const double rdet = 1.0 / detJ;
+    double sx[3] = {};  // H/HT mode scales by the mode's column
     double Ht[3][3] = {};
-    if (KIND == 1) {
-#pragma unroll
-      for (int k = 0; k < NA; ++k) {
-        double v = 2.0 * xi[kF1[k]] - 1.0;
-        if (kF2[k] >= 0) v *= 2.0 * xi[kF2[k]] - 1.0;
-        s[k] = v / detJ;
+    if (KIND == 1) {  // GL ansatz coefficients / detJ, by the lane that owns the column
+#pragma unroll 1
+      for (int k = sub; k < NA; k += 8) {
+        const int f1 = kF1[k], f2 = kF2[k];
+        double v = (q >> f1) & 1 ? 2.0 * kGaussHi - 1.0 : 2.0 * kGaussLo - 1.0;
+        if (f2 >= 0) v *= (q >> f2) & 1 ? 2.0 * kGaussHi - 1.0 : 2.0 * kGaussLo - 1.0;
+        v *= rdet;
+        sm[Cfg::O_S + 2 * k] = v;
+        sm[Cfg::O_S + 2 * k + 1] = v * a.alpha[(size_t)k * ne + e];
       }
+      __syncwarp();
     } else {
-      const double sc = detJ0 / detJ;
+      const double sc = detJ0 * rdet;
 #pragma unroll
-      for (int p = 0; p < NA; ++p) s[p] = sc * (2.0 * xi[p % 3] - 1.0);
+      for (int c = 0; c < 3; ++c) sx[c] = sc * ((q >> c) & 1 ? 2.0 * kGaussHi - 1.0 : 2.0 * kGaussLo - 1.0);
+      // Ht = A0 M A0^T with M the scaled modes
+      double T1[3][3] = {};
 #pragma unroll
-      for (int p = 0; p < NA; ++p) {
-        const int r = p / 3, c = p % 3;
-        const double w = al[p] * s[p];
+      for (int r = 0; r < 3; ++r)
 #pragma unroll
-        for (int i = 0; i < 3; ++i)
+        for (int c = 0; c < 3; ++c) {
+          const double w = a.alpha[(size_t)(3 * r + c) * ne + e] * sx[c];
 #pragma unroll
-          for (int j = 0; j < 3; ++j) Ht[i][j] += w * A0[i][r] * A0[j][c];
-      }
+          for (int i = 0; i < 3; ++i) T1[i][c] += A0[i][r] * w;
+        }
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j) Ht[i][j] = T1[i][0] * A0[j][0] + T1[i][1] * A0[j][1] + T1[i][2] * A0[j][2];
       if (KIND == 2) {
 #pragma unroll
         for (int i = 0; i < 3; ++i)
@@ -238,14 +252,13 @@ __global__ void __launch_bounds__(64) eas_element_kernel(ElemArgs a, const int32
       Ev[0] = E[0][0], Ev[1] = E[1][1], Ev[2] = E[2][2];
       Ev[3] = 2.0 * E[1][2], Ev[4] = 2.0 * E[0][2], Ev[5] = 2.0 * E[0][1];
     }
-    if (KIND == 1) {
+    if (KIND == 1) {  // lane r forms component r
+      const double* T = smem + Cfg::O_GEO + 6 * min(sub, 5);
+      double x = 0.0;
+#pragma unroll 3
+      for (int k = 0; k < NA; ++k) x += sm[Cfg::O_S + 2 * k + 1] * T[kRow[k]];
 #pragma unroll
-      for (int k = 0; k < NA; ++k) {
-        const double w = s[k] * al[k];
-        const int rr = kRow[k];
-#pragma unroll
-        for (int r = 0; r < 6; ++r) Ev[r] += w * smem[Cfg::O_GEO + 6 * r + rr];
-      }
+      for (int r = 0; r < 6; ++r) Ev[r] += __shfl_sync(0xffffffffu, x, src + r);
     }
     double S[6], Sm[3][3];
     if constexpr (HYP) {
@@ -263,6 +276,7 @@ __global__ void __launch_bounds__(64) eas_element_kernel(ElemArgs a, const int32
         S[v] = hyper::stress(pt, i, j);
         Sm[i][j] = Sm[j][i] = S[v];
       }
+#pragma unroll 1
       for (int t = sub; t < 36; t += 8) {
         const int r = t / 6, c = t % 6;
         sm[Cfg::O_C6 + t] = hyper::modulus(pt, voigt_a(r), voigt_b(r), voigt_a(c), voigt_b(c));
@@ -276,6 +290,7 @@ __global__ void __launch_bounds__(64) eas_element_kernel(ElemArgs a, const int32
         S[v] = v < 3 ? lam * trE + 2.0 * mu * Ev[v] : mu * Ev[v];
         Sm[i][j] = Sm[j][i] = S[v];
       }
+#pragma unroll 1
       for (int t = sub; t < 36; t += 8) {
         const int r = t / 6, c = t % 6;
         sm[Cfg::O_C6 + t] = (r < 3 && c < 3 ? lam : 0.0) + (r == c ? (r < 3 ? 2.0 * mu : mu) : 0.0);
@@ -301,6 +316,7 @@ __global__ void __launch_bounds__(64) eas_element_kernel(ElemArgs a, const int32
         S[v] = mu * (Jd * Ci[i][j] - Ci2[i][j]);
         Sm[i][j] = Sm[j][i] = S[v];
       }
+#pragma unroll 1
       for (int t = sub; t < 36; t += 8) {
         const int r = t / 6, c = t % 6;
         const int i = voigt_a(r), j = voigt_b(r), k = voigt_a(c), l = voigt_b(c);
@@ -325,6 +341,7 @@ __global__ void __launch_bounds__(64) eas_element_kernel(ElemArgs a, const int32
         Sm[i][j] = Sm[j][i] = S[v];
       }
       const double cc = mu - lam * lnJ;
+#pragma unroll 1
       for (int t = sub; t < 36; t += 8) {
         const int r = t / 6, c = t % 6;
         const int i = voigt_a(r), j = voigt_b(r), k = voigt_a(c), l = voigt_b(c);
@@ -366,7 +383,7 @@ __global__ void __launch_bounds__(64) eas_element_kernel(ElemArgs a, const int32
       double SdN[3];
 #pragma unroll
       for (int i = 0; i < 3; ++i) SdN[i] = Sm[i][0] * dNm[0] + Sm[i][1] * dNm[1] + Sm[i][2] * dNm[2];
-#pragma unroll
+#pragma unroll 1
       for (int d = 0; d < 5; ++d) {
         const int Jn = (sub + d) & 7;
         double dNJ[3];
@@ -388,18 +405,23 @@ __global__ void __launch_bounds__(64) eas_element_kernel(ElemArgs a, const int32
     }
 
     // enhanced-strain columns owned by this lane
+#pragma unroll 1
     for (int k = sub; k < NA; k += 8) {
       double Ea[6];
       if (KIND == 1) {
+        const double sk = sm[Cfg::O_S + 2 * k];
 #pragma unroll
-        for (int r = 0; r < 6; ++r) Ea[r] = s[k] * smem[Cfg::O_GEO + 6 * r + kRow[k]];
+        for (int r = 0; r < 6; ++r) Ea[r] = sk * smem[Cfg::O_GEO + 6 * r + kRow[k]];
       } else {
-        const int r = k / 3, c = k % 3;
+        const int r = k / 3, c = k - 3 * r;
+        const double sk = c == 0 ? sx[0] : c == 1 ? sx[1] : sx[2];
         double v[3], coef[3];
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
-          v[i] = KIND == 2 ? A0[i][r] : Fa[i][c];
-          coef[i] = s[k] * (KIND == 2 ? A0[i][c] : A0[i][r]);
+          v[i] = KIND == 2 ? smem[Cfg::O_GEO + 3 * i + r] : smem[Cfg::O_GEO + 9 + 3 * i + c];
+          coef[i] = sk * smem[Cfg::O_GEO + 3 * i + (KIND == 2 ? c : r)];
+          sm[Cfg::O_S + 6 * k + i] = v[i];
+          sm[Cfg::O_S + 6 * k + 3 + i] = coef[i];
         }
         sym_voigt(coef, v, F, Ea);
       }
@@ -417,75 +439,65 @@ __global__ void __launch_bounds__(64) eas_element_kernel(ElemArgs a, const int32
     double SdNm[3];
 #pragma unroll
     for (int i = 0; i < 3; ++i) SdNm[i] = Sm[i][0] * dNm[0] + Sm[i][1] * dNm[1] + Sm[i][2] * dNm[2];
+    double ac[3] = {};  // HT: a_c . dN0
+    if (KIND == 3) {
 #pragma unroll
-    for (int k = 0; k < NA; ++k) {
-      double t[3];
-#pragma unroll
-      for (int b = 0; b < 3; ++b) {
-        double x = 0.0;
-#pragma unroll
-        for (int r = 0; r < 6; ++r) x += sm[Cfg::O_CEA + 6 * k + r] * B[r][b];
-        t[b] = x;
-      }
-      if (KIND != 1) {
-        const int r = k / 3, c = k % 3;
-        double v[3], coef[3];
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-          v[i] = KIND == 2 ? A0[i][r] : Fa[i][c];
-          coef[i] = s[k] * (KIND == 2 ? A0[i][c] : A0[i][r]);
-        }
-        // H: v_b (coef . S dN); HT: v_b (coef . S dNm) + (F S hv)_b with hv = s a_r (a_c . dN0)
-        const double cs = coef[0] * SdNm[0] + coef[1] * SdNm[1] + coef[2] * SdNm[2];
-#pragma unroll
-        for (int b = 0; b < 3; ++b) t[b] += v[b] * cs;
-        if (KIND == 3) {
-          const double ac = A0[0][c] * dN0[0] + A0[1][c] * dN0[1] + A0[2][c] * dN0[2];
-          double hv[3], Shv[3];
-#pragma unroll
-          for (int i = 0; i < 3; ++i) hv[i] = s[k] * A0[i][r] * ac;
-#pragma unroll
-          for (int i = 0; i < 3; ++i) Shv[i] = Sm[i][0] * hv[0] + Sm[i][1] * hv[1] + Sm[i][2] * hv[2];
-#pragma unroll
-          for (int b = 0; b < 3; ++b) t[b] += F[b][0] * Shv[0] + F[b][1] * Shv[1] + F[b][2] * Shv[2];
-        }
-      }
-#pragma unroll
-      for (int b = 0; b < 3; ++b) share[8 * (kL + 24 * k + 3 * sub + b)] = w * t[b];
+      for (int c = 0; c < 3; ++c) ac[c] = A0[0][c] * dN0[0] + A0[1][c] * dN0[1] + A0[2][c] * dN0[2];
     }
-    // D share: (E_alpha^T C E_alpha + E_alpha,alpha) w detJ (enhancedassumedstrains.hh:400)
+#pragma unroll 1
+    for (int k0 = 0; k0 < NA; k0 += 3)
 #pragma unroll
-    for (int m = 0; m < Cfg::DSH; ++m) {
-      const int t = sub + 8 * m;
-      if (t < Cfg::NT) {
-        int aa, bb;
-        packed_index(t, NA, aa, bb);
-        double x = 0.0;
+      for (int c = 0; c < 3; ++c) {
+        const int k = k0 + c;
+        double t[3];
 #pragma unroll
-        for (int r = 0; r < 6; ++r) x += sm[Cfg::O_EA + 6 * aa + r] * sm[Cfg::O_CEA + 6 * bb + r];
-        if (KIND != 1) {  // (v^a . v^b)(coef^a . S coef^b)  (displacementgradient.hh:213-230)
-          const int ra = aa / 3, ca = aa % 3, rb = bb / 3, cb = bb % 3;
-          double va[3], vb[3], fa[3], fb[3];
+        for (int b = 0; b < 3; ++b) {
+          double x = 0.0;
 #pragma unroll
-          for (int i = 0; i < 3; ++i) {
-            va[i] = KIND == 2 ? A0[i][ra] : Fa[i][ca];
-            vb[i] = KIND == 2 ? A0[i][rb] : Fa[i][cb];
-            fa[i] = s[aa] * (KIND == 2 ? A0[i][ca] : A0[i][ra]);
-            fb[i] = s[bb] * (KIND == 2 ? A0[i][cb] : A0[i][rb]);
-          }
-          double Sfb[3];
-#pragma unroll
-          for (int i = 0; i < 3; ++i) Sfb[i] = Sm[i][0] * fb[0] + Sm[i][1] * fb[1] + Sm[i][2] * fb[2];
-          x += (va[0] * vb[0] + va[1] * vb[1] + va[2] * vb[2]) * (fa[0] * Sfb[0] + fa[1] * Sfb[1] + fa[2] * Sfb[2]);
+          for (int r = 0; r < 6; ++r) x += sm[Cfg::O_CEA + 6 * k + r] * B[r][b];
+          t[b] = x;
         }
-        share[8 * (kD + t)] = w * x;
+        if (KIND != 1) {
+          const double* v = sm + Cfg::O_S + 6 * k;
+          const double* coef = v + 3;
+          // H: v_b (coef . S dN); HT: v_b (coef . S dNm) + (F S hv)_b with hv = s a_r (a_c . dN0)
+          const double cs = coef[0] * SdNm[0] + coef[1] * SdNm[1] + coef[2] * SdNm[2];
+#pragma unroll
+          for (int b = 0; b < 3; ++b) t[b] += v[b] * cs;
+          if (KIND == 3) {
+            double hv[3], Shv[3];
+#pragma unroll
+            for (int i = 0; i < 3; ++i) hv[i] = coef[i] * ac[c];
+#pragma unroll
+            for (int i = 0; i < 3; ++i) Shv[i] = Sm[i][0] * hv[0] + Sm[i][1] * hv[1] + Sm[i][2] * hv[2];
+#pragma unroll
+            for (int b = 0; b < 3; ++b) t[b] += F[b][0] * Shv[0] + F[b][1] * Shv[1] + F[b][2] * Shv[2];
+          }
+        }
+#pragma unroll
+        for (int b = 0; b < 3; ++b) share[8 * (kL + 24 * k + 3 * sub + b)] = w * t[b];
       }
+    // D share: (E_alpha^T C E_alpha + E_alpha,alpha) w detJ (enhancedassumedstrains.hh:400)
+#pragma unroll 1
+    for (int t = sub; t < Cfg::NT; t += 8) {
+      int aa, bb;
+      packed_index(t, NA, aa, bb);
+      double x = 0.0;
+#pragma unroll
+      for (int r = 0; r < 6; ++r) x += sm[Cfg::O_EA + 6 * aa + r] * sm[Cfg::O_CEA + 6 * bb + r];
+      if (KIND != 1) {  // (v^a . v^b)(coef^a . S coef^b)  (displacementgradient.hh:213-230)
+        const double *va = sm + Cfg::O_S + 6 * aa, *vb = sm + Cfg::O_S + 6 * bb, *fa = va + 3, *fb = vb + 3;
+        double Sfb[3];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) Sfb[i] = Sm[i][0] * fb[0] + Sm[i][1] * fb[1] + Sm[i][2] * fb[2];
+        x += (va[0] * vb[0] + va[1] * vb[1] + va[2] * vb[2]) * (fa[0] * Sfb[0] + fa[1] * Sfb[1] + fa[2] * Sfb[2]);
+      }
+      share[8 * (kD + t)] = w * x;
     }
     // R~ share: E_alpha^T S w detJ (enhancedassumedstrains.hh:428)
-#pragma unroll
-    for (int m = 0; m < Cfg::RSH; ++m) {
-      const int k = sub + 8 * m;
-      if (k < NA) {
+    if (WANT_R) {
+#pragma unroll 1
+      for (int k = sub; k < NA; k += 8) {
         double x = 0.0;
 #pragma unroll
         for (int r = 0; r < 6; ++r) x += sm[Cfg::O_EA + 6 * k + r] * S[r];
@@ -495,46 +507,45 @@ __global__ void __launch_bounds__(64) eas_element_kernel(ElemArgs a, const int32
   }
   __syncthreads();
 
-  // ---- sums over the points, in their order ---------------------------------------------------------------
+  // ---- sums over the points, in a fixed order ---------------------------------------------------------------
   const double* shares = smem + Cfg::O_SHARE;
   auto total = [&](int t) {
-    double x = shares[8 * t];
-#pragma unroll
-    for (int p = 1; p < 8; ++p) x += shares[8 * t + p];
-    return x;
+    const double* x = shares + 8 * t;
+    return ((x[0] + x[1]) + (x[2] + x[3])) + ((x[4] + x[5]) + (x[6] + x[7]));
   };
   double* L = smem + Cfg::O_L;
   double* D = smem + Cfg::O_D;
   double* Y = smem + Cfg::O_Y;
   int* perm = reinterpret_cast<int*>(smem + Cfg::O_PERM);
+#pragma unroll 1
   for (int t = threadIdx.x; t < 24 * NA; t += 64) L[t] = total(kL + t);
+#pragma unroll 1
   for (int t = threadIdx.x; t < Cfg::NT; t += 64) {
     int aa, bb;
     packed_index(t, NA, aa, bb);
     D[NA * aa + bb] = D[NA * bb + aa] = total(kD + t);
   }
   if (threadIdx.x < NA) {
-    smem[Cfg::O_RT + threadIdx.x] = total(kR + threadIdx.x);
+    if (WANT_R) smem[Cfg::O_RT + threadIdx.x] = total(kR + threadIdx.x);
     perm[threadIdx.x] = threadIdx.x;
   }
   __syncthreads();
 
   // ---- static condensation ------------------------------------------------------------------------------
   if (threadIdx.x < 32) {
-    // LU with partial pivoting of D in place: lane i holds row i
+    // LU with partial pivoting of D in place
+    double* rpiv = smem + Cfg::O_INV;
+#pragma unroll 1
     for (int k = 0; k < NA; ++k) {
-      double best = lane >= k && lane < NA ? fabs(D[NA * lane + k]) : -1.0;
-      const bool nan = __any_sync(0xffffffffu, best != best);  // as a singular pivot, decided by all lanes alike
-      int p = lane;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {  // the largest, of equal ones the first row
-        const double v = __shfl_xor_sync(0xffffffffu, best, o);
-        const int w = __shfl_xor_sync(0xffffffffu, p, o);
-        if (v > best || (v == best && w < p)) best = v, p = w;
-      }
-      if (nan || !(best > 0.0)) {
+      // the largest magnitude, of equal ones the first row: magnitudes are ordered as their bits
+      const bool cand = lane >= k && lane < NA;
+      const unsigned long long m = (unsigned long long)__double_as_longlong(fabs(cand ? D[NA * lane + k] : 0.0));
+      const unsigned hi = (unsigned)(m >> 32), H = __reduce_max_sync(0xffffffffu, hi);
+      const unsigned lo = hi == H ? (unsigned)m : 0u, Lo = __reduce_max_sync(0xffffffffu, lo);
+      const int p = __ffs(__ballot_sync(0xffffffffu, cand && hi == H && lo == Lo)) - 1;
+      if ((H | Lo) == 0u || H > 0x7ff00000u || (H == 0x7ff00000u && Lo != 0u)) {  // zero or NaN
         bad |= kStatusSingularD;
-        if (lane == 0) D[NA * k + k] = 1.0;
+        if (lane == 0) D[NA * k + k] = rpiv[k] = 1.0;
         __syncwarp();
         continue;
       }
@@ -552,15 +563,19 @@ __global__ void __launch_bounds__(64) eas_element_kernel(ElemArgs a, const int32
         __syncwarp();
       }
       const double inv = 1.0 / D[NA * k + k];
-      if (lane > k && lane < NA) {
-        const double l = D[NA * lane + k] * inv;
-        D[NA * lane + k] = l;
-        for (int j = k + 1; j < NA; ++j) D[NA * lane + j] -= l * D[NA * k + j];
+      if (lane == 0) rpiv[k] = inv;
+      if (lane > k && lane < NA) D[NA * lane + k] *= inv;
+      __syncwarp();
+#pragma unroll 1
+      for (int i = k + 1 + (lane >> 3); i < NA; i += 4) {  // eight lanes a row
+        const double l = D[NA * i + k];
+#pragma unroll 1
+        for (int j = k + 1 + (lane & 7); j < NA; j += 8) D[NA * i + j] -= l * D[NA * k + j];
       }
       __syncwarp();
     }
     // columns of D^{-1} L (lanes 0 .. 23) and D^{-1} R~ (lane 24)
-    if (lane < 25) {
+    if (lane < (WANT_R ? 25 : 24)) {
       double z[NA];
 #pragma unroll
       for (int k = 0; k < NA; ++k) z[k] = lane < 24 ? L[24 * perm[k] + lane] : smem[Cfg::O_RT + perm[k]];
@@ -572,7 +587,7 @@ __global__ void __launch_bounds__(64) eas_element_kernel(ElemArgs a, const int32
       for (int i = NA - 1; i >= 0; --i) {
 #pragma unroll
         for (int j = i + 1; j < NA; ++j) z[i] -= D[NA * i + j] * z[j];
-        z[i] /= D[NA * i + i];
+        z[i] *= rpiv[i];
       }
       double* out = lane < 24 ? Y + lane * NA : smem + Cfg::O_RT + NA;
 #pragma unroll
@@ -603,6 +618,7 @@ __global__ void __launch_bounds__(64) eas_element_kernel(ElemArgs a, const int32
     }
   } else {
     double* out = a.elem_mat + 576 * (size_t)li;
+#pragma unroll 1
     for (int t = threadIdx.x; t < 360; t += 64) {
       const int d = t / 72, I = (t / 9) & 7, i = (t % 9) / 3, j = t % 3, J = (I + d) & 7;
       double x = 0.0;
