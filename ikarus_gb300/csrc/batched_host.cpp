@@ -214,27 +214,33 @@ static void batched_cg(ikr_nr nr, ikr_fes f, ikr_asm a, const std::vector<uint8_
   std::vector<int32_t> flag(ni), its(ni);
   int chunk = std::max(1, P.first_chunk);
   bool first = true;
-  // the planner's own choice runs as the one-reduction kernel where that fits and no other solver shares the device; the
-  // launches count as the planner's variant
-  const bool halo = P.variant == -1 && P.share >= 1.0 && plan_halo_launch(nr, f, a, a->fp32, run);
-  // the one-reduction kernel is re-planned more often: the CTAs of finished instances idle until the launch ends, which
+  // the planner's own choice runs as the one-reduction kernel where that fits and no other solver shares the device (with
+  // more instances than SMs from the launch on at which few enough are left); the launches count as the planner's variant
+  bool halo = false;
+  // it is re-planned more often than the other kernels, at most 256 iterations a launch: the CTAs of finished instances idle until the launch ends, which
   // at six microseconds per iteration costs more than a launch (128 instances, FP32: 119 / 117 / 121 / 123 ms at most
   // 128 / 256 / 512 / 1 024 iterations; 100 instances, FP64: 380 / 383 / 397 / 397 ms)
-  const int longest = halo ? 256 : 4096;
   while (!run.empty()) {
+    ikr::HaloStart start = ikr::HaloStart::kContinue;
+    if (halo) {
+      need(plan_halo_launch(nr, f, a, a->fp32, run), IKR_ERR_ARG, "the batched CG's split does not fit");
+    } else if (P.variant == -1 && P.share >= 1.0 && plan_halo_launch(nr, f, a, a->fp32, run)) {
+      halo = true;
+      start = first ? ikr::HaloStart::kFirst : ikr::HaloStart::kTakeOver;
+    }
     if (halo) {
       std::vector<int> order;
       P.cur_variant = planned(nr, f, a, a->fp32, run, order).variant;
-      need(first || plan_halo_launch(nr, f, a, a->fp32, run), IKR_ERR_ARG, "the batched CG's split does not fit");
+      chunk = std::min(chunk, std::max(256, P.first_chunk));
     } else {
       plan_batch_launch(nr, f, a, a->fp32, run);
     }
     if (halo) {
       CK(ikr::launch_batched_halo(a->bsr(), w, P.halo_split, P.halo_cnt.p, P.halo_rows.p, P.col16.p, P.max_rows,
                                   nr->rhs.p, nr->corr.p, f->inst_off.p, P.cta_inst.p, P.cta_first.p, P.cta_size.p,
-                                  nr->inst_rtol.p, st.linear_max_iter, chunk, first, P.st.p, nr->inst_cg_iters.p,
+                                  nr->inst_rtol.p, st.linear_max_iter, chunk, start, P.st.p, nr->inst_cg_iters.p,
                                   P.flag.p, ni, nr->inst_cg_res.p, s));
-      count(first ? 2 : 1);
+      count(start == ikr::HaloStart::kContinue ? 1 : 2);
     } else if (P.cur_variant == 4)
       CK(ikr::launch_batched_pcg_cluster(a->bsr(), w.minv, nr->rhs.p, nr->corr.p, P.n_cta, f->inst_off.p,
                                          P.cta_inst.p, w.x, w.r, w.z, w.p0, w.p1, nr->inst_rtol.p, st.linear_max_iter,
@@ -250,7 +256,7 @@ static void batched_cg(ikr_nr nr, ikr_fes f, ikr_asm a, const std::vector<uint8_
     ++P.launches;
     ++P.launches_by_variant[P.cur_variant];
     first = false;
-    chunk = std::min(2 * chunk, std::max(chunk, longest));
+    chunk = std::min(2 * chunk, std::max(chunk, halo ? 256 : 4096));
     P.flag.download(flag.data(), ni, s);
     CK(cudaStreamSynchronize(s));
     std::vector<int> next;

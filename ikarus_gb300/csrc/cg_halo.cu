@@ -923,6 +923,24 @@ __global__ void __launch_bounds__(512) halo_groups_init_kernel(HaloGroups g, con
   }
 }
 
+// GROUPS: from the state that the kernels of batched.cu leave between launches (p_old in p0 or p1 by the parity of the
+// iteration, beta in st) to this form's: p = z + beta p_old, no published rows.  One CTA per instance.
+template <typename T>
+__global__ void __launch_bounds__(512) halo_groups_take_over_kernel(HaloGroups g, const T* __restrict__ z, T* published) {
+  if (g.first[blockIdx.x] != (int)blockIdx.x) return;
+  const int inst = g.inst[blockIdx.x];
+  T* p = static_cast<T*>(g.p);
+  const T beta = T(g.st[4 * inst + 3]);
+  const bool in_p = g.its[inst] & 1;
+  for (int64_t i = g.node_off[inst] + threadIdx.x; i < g.node_off[inst + 1]; i += blockDim.x)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const T old = in_p ? p[4 * i + c] : published[4 * i + c];
+      if (c < 3) p[4 * i + c] = z[4 * i + c] + beta * old;
+      published[4 * i + c] = T(0);
+    }
+}
+
 // Shared-memory layout and eligibility of a variant on a system.  Rows per thread and the shared memory of p, the
 // partial products and the halo list bound the size: about 250 k rows of a structured mesh in FP32, 150 k in FP64.
 struct Layout {
@@ -1087,7 +1105,7 @@ bool batched_halo_fits(const HaloPlan& P, bool fp32) {
 cudaError_t launch_batched_halo(const Bsr& A, const PcgWork& work, const HaloPlan& P, int32_t* cnt, int32_t* halo,
                                 uint16_t* col16, int max_rows, const double* b, double* x_out, const int32_t* node_off,
                                 const int32_t* cta_inst, const int32_t* cta_first, const int32_t* cta_size,
-                                const double* rtol, int max_iter, int chunk, bool first_launch, double* st, int32_t* its,
+                                const double* rtol, int max_iter, int chunk, HaloStart start, double* st, int32_t* its,
                                 int32_t* flag, int n_inst, double* relres, cudaStream_t s) {
   const Layout L = work.fp32 ? layout_of<float>(P, warps_of(true, 0)) : layout_of<double>(P, warps_of(false, 0));
   if (!L.ok) return cudaErrorInvalidConfiguration;
@@ -1100,10 +1118,14 @@ cudaError_t launch_batched_halo(const Bsr& A, const PcgWork& work, const HaloPla
   if (e == cudaSuccess) e = cudaMemsetAsync(flag, 0x7f, sizeof(int32_t) * n_inst, s);
   if (e != cudaSuccess) return e;
   halo_plan_kernel<true><<<P.n_cta, 1024, (max_rows + 31) / 32 * 8, s>>>(A, P, g, nullptr, cnt, halo, col16);
-  if (first_launch && w.fp32)
+  if (start == HaloStart::kTakeOver && w.fp32)
+    halo_groups_take_over_kernel<float><<<P.n_cta, 512, 0, s>>>(g, (const float*)w.z, (float*)w.p1);
+  else if (start == HaloStart::kTakeOver)
+    halo_groups_take_over_kernel<double><<<P.n_cta, 512, 0, s>>>(g, (const double*)w.z, (double*)w.p1);
+  else if (start == HaloStart::kFirst && w.fp32)
     halo_groups_init_kernel<float><<<P.n_cta, 512, 0, s>>>(g, b, (const float*)w.minv, (float*)w.x, (float*)w.r,
                                                           (float*)w.z, (float*)w.p1);
-  else if (first_launch)
+  else if (start == HaloStart::kFirst)
     halo_groups_init_kernel<double><<<P.n_cta, 512, 0, s>>>(g, b, (const double*)w.minv, (double*)w.x, (double*)w.r,
                                                            (double*)w.z, (double*)w.p1);
   e = cudaGetLastError();

@@ -18,6 +18,7 @@ CASES = [
     (140, (6, 6), (8, 8), False),   # 567 rows: two passes in FP32, three in FP64
     (140, (12, 12), (8, 8), False), # 1 053 rows: three passes in FP32; FP64 does not fit and keeps the row loop
     (160, (1, 2), (1, 1), False),   # more instances than SMs: no split
+    (300, (1, 9), (1, 2), False),   # no split at first, then the instances left over are taken over
 ]
 
 
