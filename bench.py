@@ -442,7 +442,8 @@ def finish(args, p, world, t_mixed, t_e2e, t_plain, plain_info, infos, launches,
     persistent = kind >= 5
     if persistent:
         bpl += 9 * n_nodes * 4
-    kname = ("pcg_persistent_kernel<float> (per CG iteration)" if persistent else
+    kname = (("pcg_halo_kernel<float>" if kind in (12, 13) else "pcg_persistent_kernel<float>") + " (per CG iteration)"
+             if persistent else
              "pcg_spmv_staged_kernel<float>" if kind > 0 else "pcg_spmv_kernel<float>")
     # per launch: a persistent launch is one CG solve (spmv_n counts its iterations), a staged launch one SpMV
     n_launch = max(prof_solves, 1) if persistent else max(spmv_n, 1)

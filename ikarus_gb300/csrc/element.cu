@@ -13,9 +13,11 @@
 // and the internal force f_I = w [ mu F grad N_I + (lambda ln J - mu) g_I ] equals B_I^T S w.
 // Lane I owns the node blocks (I, I+d mod 8), d = 0..4, and writes d = 1..3 also transposed, so each of the
 // 64 blocks is produced once and the element matrix is exactly symmetric.
-// Assembly is a plain read-modify-write into the BSR values through the precomputed element-to-block slot map;
-// the host launches one colour class at a time (no two elements of a class share a node), so the summation
-// order is fixed and repeated runs are bit-identical.
+// This node-per-lane kernel forms the FP32 tangents, energies and the FP64 element matrices of the other laws; the FP64
+// residual and Neo-Hooke tangent have kernels with a Gauss point per lane.  Assembly gathers element vectors, blocks or
+// matrices in ascending element order; the FP32 tangent's coloured form is a plain read-modify-write into the BSR values
+// through the element-to-block slot map, one colour class at a time (no two elements of a class share a node).  Either way the
+// summation order is fixed and repeated runs are bit-identical.
 #include <cmath>
 #include <type_traits>
 
@@ -1155,7 +1157,7 @@ void launch_disp_t(const ElemArgs& a, const int32_t* list, int n_list, int e_bas
 }  // namespace
 
 void launch_row_tangent(const ElemArgs& a, const int32_t* ne_ptr, const int32_t* ne_elems, cudaStream_t s) {
-  // FP32 only: the FP64 form of this kernel exceeds the register file (the coloured element kernel assembles it)
+  // FP32 only: the FP64 form of this kernel exceeds the register file
   row_tangent_kernel<float><<<(a.n_nodes + 127) / 128, 128, 0, s>>>(a, ne_ptr, ne_elems);
 }
 
@@ -1163,7 +1165,7 @@ void launch_disp_element(const ElemArgs& a, int mode, bool fp32_tangent, const i
                          cudaStream_t s) {
   if (n_list <= 0) return;
   switch (mode) {
-    case kWantR | kElemOut:  // Gauss-point-per-lane kernel (its shared exchange fits up to 32 per block)
+    case kWantR | kElemOut:  // Gauss-point-per-lane kernel
       // one warp per block while that does not fill the SMs' warp slots: a block's warps share one FP64 pipe
       if (n_list <= 4096) launch_residual_gp<4>(a, list, n_list, e_base, s);
       else if (a.epb == 16) launch_residual_gp<16>(a, list, n_list, e_base, s);

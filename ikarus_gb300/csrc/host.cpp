@@ -80,8 +80,8 @@ void need(bool c, int code, const char* msg) {
 uint64_t cache_key(ikr_req r, ikr_fes f) { return (r->id * 0x9E3779B97F4A7C15ull) ^ (r->version << 20) ^ f->alpha_version; }
 
 // Elements per block of the displacement element kernel: each of 16, 32 and 64 is timed once on a complete
-// coloured pass of the given kind and the fastest is kept for the element set (the choice does not change any
-// result: the summation order into each block is fixed by the colouring).  `pass` runs one pass with args.epb.
+// pass of the given kind and the fastest is kept for the element set (the choice does not change any
+// result: the summation order does not depend on it).  `pass` runs one pass with args.epb.
 template <typename Pass>
 static int choose_epb(ikr_fes f, Pass pass) {
   if (f->na > 0) return 32;  // the EAS kernel has its own launch shape

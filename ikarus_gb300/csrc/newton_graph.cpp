@@ -2,7 +2,7 @@
 //
 // Launched one by one, an iteration of the mixed form is about 25 launches with five host round trips (status after
 // the tangent, the CG scalars, the correction norm, status after the residual, the residual norm).  Captured once,
-// the same launches -- tangent assembly (one launch per colour class, the row kernel or element blocks + gather,
+// the same launches -- tangent assembly (element blocks or matrices and gather, the row kernel or one launch per colour class,
 // manipulator entries), block-Jacobi inverse, right-hand side, CG init, the persistent cooperative CG, the
 // correction, its norm, u += correction, residual assembly, its norm -- and the copies of the norms, the CG scalars
 // and the element status into pinned host memory run as one graph launch followed by one synchronisation.  The

@@ -486,7 +486,10 @@ int ikr_newton_instance_linear_iterations(ikr_nr nr, int64_t* cg_iterations);
  * FP32 one instance per 16-CTA thread-block cluster with vectors in distributed shared memory; sixteen (FP64 only),
  * eight or four threads per row with the matrix in shared memory; one row per thread; rows looped per thread); 0..5
  * keeps variant 0 (row loop), 1 (one row per thread), 2 (four threads per row), 3 (eight), 4 (clusters, FP32) or 5
- * (sixteen threads per row) where it fits, else the row loop.  For tests and tuning; the results agree to rounding.  batched_cg_launches: launches since creation. */
+ * (sixteen threads per row) where it fits, else the row loop.  A launch planned with -1 runs as groups of the
+ * one-reduction CG (at most 256 iterations unless first_chunk is larger) where its split fits and no other solver shares
+ * the device, counted under the planner's variant.  For tests and tuning; the results agree to rounding.
+ * batched_cg_launches: launches since creation. */
 int ikr_newton_set_batched_cg(ikr_nr nr, int32_t variant, int32_t first_chunk);
 int ikr_newton_batched_cg_launches(ikr_nr nr, int64_t* n);
 /* the same per kernel variant 0..5 (six values) */
