@@ -762,12 +762,13 @@ int ikr_assembler_vector(ikr_asm a, ikr_req r, int32_t aff, int32_t dbc, double*
     need(dbc >= 0 && dbc <= 2, IKR_ERR_ARG, "invalid DBCOption");
     assemble_vector(a, r, dbc == IKR_DBC_RAW ? IKR_DBC_RAW : IKR_DBC_FULL);
     if (!out) return;
-    std::vector<double> full(a->n);
-    a->R.download(full.data(), full.size(), a->fes->stream);
-    CK(cudaStreamSynchronize(a->fes->stream));
-    if (dbc != IKR_DBC_REDUCED) {
-      std::copy(full.begin(), full.end(), out);
+    if (dbc != IKR_DBC_REDUCED) {  // straight into the caller's array: a host vector between cost a fifth of a 3 MB call
+      a->R.download(out, a->n, a->fes->stream);
+      CK(cudaStreamSynchronize(a->fes->stream));
     } else {  // getReducedVectorImpl (simpleassemblers.inl:96-118): free dofs in order
+      std::vector<double> full(a->n);
+      a->R.download(full.data(), full.size(), a->fes->stream);
+      CK(cudaStreamSynchronize(a->fes->stream));
       int k = 0;
       for (int i = 0; i < a->n; ++i)
         if (!a->fixed_h[i]) out[k++] = full[i];
