@@ -376,7 +376,7 @@ __global__ void __launch_bounds__(EPB * 8) disp_element_kernel(ElemArgs a, const
   if (WANT_E && ELEM_OUT && sub == 0) a.elem_energy[li] = psi_tot;
   if constexpr (BLOCKS) {
     // lane I's blocks (I, I + d), d = 0..3, and (I, I + 4) for I < 4, into the warp's stage, then the element's 324
-    // values to blk[e] (8 lanes, 16 bytes each per store)
+    // values to blk of its place in the launch (8 lanes, 16 bytes each per store)
     KT* st = stage[threadIdx.x >> 5] + (es & 3) * (kElemBlockCount * 9);
 #pragma unroll
     for (int d = 0; d < 5; ++d) {
@@ -389,7 +389,7 @@ __global__ void __launch_bounds__(EPB * 8) disp_element_kernel(ElemArgs a, const
     }
     __syncwarp(0xFFu << (lane & ~7));
     const float4* src4 = reinterpret_cast<const float4*>(st);
-    float4* dst4 = reinterpret_cast<float4*>(static_cast<float*>(a.blk) + (size_t)e * (kElemBlockCount * 9));
+    float4* dst4 = reinterpret_cast<float4*>(static_cast<float*>(a.blk) + (size_t)li * (kElemBlockCount * 9));
     for (int k = sub; k < kElemBlockCount * 9 / 4; k += 8) dst4[k] = src4[k];
   } else if (WANT_K) {
     if (ELEM_OUT) {
@@ -894,7 +894,7 @@ __global__ void __launch_bounds__(32) tangent64_kernel(ElemArgs a, int n_list, i
     __syncwarp();
     if (!active) return;
     const double2* s2 = reinterpret_cast<const double2*>(st);
-    double2* d2 = reinterpret_cast<double2*>(static_cast<double*>(a.blk) + (size_t)e * (kElemBlockCount * 9));
+    double2* d2 = reinterpret_cast<double2*>(static_cast<double*>(a.blk) + (size_t)li * (kElemBlockCount * 9));
     for (int k = sub; k < kElemBlockCount * 9 / 2; k += 8) d2[k] = s2[k];
   }
 }
@@ -1026,21 +1026,22 @@ __global__ void tangent_inv_count_kernel(const int32_t* __restrict__ slot, int64
   const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (t < n) atomicAdd(&cnt[slot[t]], 1);
 }
-__global__ void tangent_inv_fill_kernel(const int32_t* __restrict__ slot, int ne, const int32_t* __restrict__ ptr,
-                                        int32_t* __restrict__ cursor, int32_t* __restrict__ inv) {
+// (codes and offsets are unsigned: up to 67 million elements)
+__global__ void tangent_inv_fill_kernel(const int32_t* __restrict__ slot, int ne, const uint32_t* __restrict__ ptr,
+                                        int32_t* __restrict__ cursor, uint32_t* __restrict__ inv) {
   const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (t >= 64LL * ne) return;
   const int pair = (int)(t / ne), e = (int)(t % ne);
   const int b = slot[t];
-  inv[ptr[b] + atomicAdd(&cursor[b], 1)] = e * 64 + pair;
+  inv[ptr[b] + (uint32_t)atomicAdd(&cursor[b], 1)] = (uint32_t)e * 64u + (uint32_t)pair;
 }
-__global__ void tangent_inv_sort_kernel(const int32_t* __restrict__ ptr, int32_t* __restrict__ inv, int64_t n) {
+__global__ void tangent_inv_sort_kernel(const uint32_t* __restrict__ ptr, uint32_t* __restrict__ inv, int64_t n) {
   const int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (b >= n) return;
-  const int c0 = ptr[b], c1 = ptr[b + 1];
-  for (int i = c0 + 1; i < c1; ++i) {  // at most 8 entries: insertion sort, ascending
-    const int v = inv[i];
-    int j = i - 1;
+  const int64_t c0 = ptr[b], c1 = ptr[b + 1];
+  for (int64_t i = c0 + 1; i < c1; ++i) {  // at most 8 entries: insertion sort, ascending
+    const uint32_t v = inv[i];
+    int64_t j = i - 1;
     while (j >= c0 && inv[j] > v) {
       inv[j + 1] = inv[j];
       --j;
@@ -1055,10 +1056,11 @@ __global__ void tangent_inv_sort_kernel(const int32_t* __restrict__ ptr, int32_t
 // element blocks), rounded to T once.
 template <typename T, typename S, bool FULL>
 __global__ void __launch_bounds__(256) tangent_gather_kernel(Bsr A, const int32_t* __restrict__ gslice,
-                                                             const int32_t* __restrict__ ptr,
-                                                             const int32_t* __restrict__ inv,
+                                                             const uint32_t* __restrict__ ptr,
+                                                             const uint32_t* __restrict__ inv,
                                                              const S* __restrict__ blk,
-                                                             const uint8_t* __restrict__ nf, T* __restrict__ val) {
+                                                             const uint8_t* __restrict__ nf, T* __restrict__ val,
+                                                             int e0, int n) {
   const int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (b >= A.n_padded) return;
   const int g = (int)(b >> 5), l = (int)(b & 31);
@@ -1066,9 +1068,16 @@ __global__ void __launch_bounds__(256) tangent_gather_kernel(Bsr A, const int32_
   S acc[9];
 #pragma unroll
   for (int k = 0; k < 9; ++k) acc[k] = S(0);
-  const int c0 = ptr[b], c1 = ptr[b + 1];
-  for (int c = c0; c < c1; ++c) {
-    const int code = __ldg(inv + c), e = code >> 6, I = (code >> 3) & 7, J = code & 7;
+  const uint32_t c0 = ptr[b], c1 = ptr[b + 1];
+  T* out = val + (size_t)g * 288 + l;
+  if (e0 > 0) {  // a later part of the elements: on top of the former parts' sums
+#pragma unroll
+    for (int k = 0; k < 9; ++k) acc[k] = S(out[32 * k]);
+  }
+  for (uint32_t c = c0; c < c1; ++c) {
+    const uint32_t code = __ldg(inv + c);
+    const int e = (int)(code >> 6) - e0, I = (code >> 3) & 7, J = code & 7;
+    if ((unsigned)e >= (unsigned)n) continue;
     S v[9];
     if constexpr (FULL) {
       const S* src = blk + (size_t)e * 576 + 72 * J + 3 * I;
@@ -1095,7 +1104,6 @@ __global__ void __launch_bounds__(256) tangent_gather_kernel(Bsr A, const int32_
   uint8_t fr = 0, fc = 0;
   const int col = A.col_sell[b];
   if (nf && c1 > c0) fr = nf[row], fc = nf[col];
-  T* out = val + (size_t)g * 288 + l;
 #pragma unroll
   for (int i = 0; i < 3; ++i)
 #pragma unroll
@@ -1194,23 +1202,26 @@ void launch_tangent_inverse_count(const int32_t* slot, int n_elems, int32_t* cnt
 void launch_tangent_inverse_fill(const int32_t* slot, int n_elems, const int32_t* ptr, int32_t* cursor, int32_t* inv,
                                  int64_t n_padded, cudaStream_t s) {
   const int64_t n = 64LL * n_elems;
-  if (n > 0) tangent_inv_fill_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(slot, n_elems, ptr, cursor, inv);
-  if (n_padded > 0) tangent_inv_sort_kernel<<<(unsigned)((n_padded + 255) / 256), 256, 0, s>>>(ptr, inv, n_padded);
+  if (n > 0) tangent_inv_fill_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(
+                 slot, n_elems, (const uint32_t*)ptr, cursor, (uint32_t*)inv);
+  if (n_padded > 0)
+    tangent_inv_sort_kernel<<<(unsigned)((n_padded + 255) / 256), 256, 0, s>>>((const uint32_t*)ptr, (uint32_t*)inv,
+                                                                              n_padded);
 }
 template <typename T, typename S, bool FULL>
 static void gather_t(const Bsr& A, const int32_t* gslice, const int32_t* inv_ptr, const int32_t* inv, const void* blk,
-                     const uint8_t* nf, void* val, cudaStream_t s) {
+                     const uint8_t* nf, void* val, int e0, int n, cudaStream_t s) {
   tangent_gather_kernel<T, S, FULL><<<(unsigned)((A.n_padded + 255) / 256), 256, 0, s>>>(
-      A, gslice, inv_ptr, inv, (const S*)blk, nf, (T*)val);
+      A, gslice, (const uint32_t*)inv_ptr, (const uint32_t*)inv, (const S*)blk, nf, (T*)val, e0, n);
 }
 void launch_tangent_gather(const Bsr& A, bool fp32_val, bool fp32_blk, bool full, const int32_t* gslice,
                            const int32_t* inv_ptr, const int32_t* inv, const void* blk, const uint8_t* node_fixed,
-                           void* val, cudaStream_t s) {
+                           void* val, int e0, int n, cudaStream_t s) {
   if (A.n_padded <= 0) return;
-  if (fp32_blk) gather_t<float, float, false>(A, gslice, inv_ptr, inv, blk, node_fixed, val, s);
-  else if (full && fp32_val) gather_t<float, double, true>(A, gslice, inv_ptr, inv, blk, node_fixed, val, s);
-  else if (full) gather_t<double, double, true>(A, gslice, inv_ptr, inv, blk, node_fixed, val, s);
-  else gather_t<double, double, false>(A, gslice, inv_ptr, inv, blk, node_fixed, val, s);
+  if (fp32_blk) gather_t<float, float, false>(A, gslice, inv_ptr, inv, blk, node_fixed, val, e0, n, s);
+  else if (full && fp32_val) gather_t<float, double, true>(A, gslice, inv_ptr, inv, blk, node_fixed, val, e0, n, s);
+  else if (full) gather_t<double, double, true>(A, gslice, inv_ptr, inv, blk, node_fixed, val, e0, n, s);
+  else gather_t<double, double, false>(A, gslice, inv_ptr, inv, blk, node_fixed, val, e0, n, s);
 }
 void launch_node_corners(const int32_t* conn, int n_elems, int n_nodes, const int32_t* ptr, int32_t* codes,
                          cudaStream_t s) {

@@ -189,13 +189,18 @@ static void assemble_matrix32(ikr_asm a, ikr::ElemArgs& args, const uint8_t* nf)
   const bool row_ok = f->material == 0 && f->n_inst == 0;
   auto element_blocks = [&]() {
     a->build_gather_map();
-    a->eblk.alloc((size_t)f->ne * ikr::kElemBlockCount * 9);
+    constexpr int kPer = ikr::kElemBlockCount * 9;
+    const int part = a->gather_part(f->ne, sizeof(float) * kPer);
+    a->eblk.alloc((size_t)part * kPer);
     ikr::ElemArgs t = args;
     t.blk = a->eblk.p;
-    f->launch_elements(t, ikr::kWantK | ikr::kElemBlocks, true, nullptr, f->ne, 0);
-    ikr::launch_tangent_gather(a->bsr(), true, true, false, a->gslice.p, a->inv_ptr.p, a->inv_idx.p, a->eblk.p, nf,
-                               a->values(), f->stream);
-    count(1);
+    for (int e0 = 0; e0 < f->ne; e0 += part) {
+      const int n = std::min(part, f->ne - e0);
+      f->launch_elements(t, ikr::kWantK | ikr::kElemBlocks, true, nullptr, n, e0);
+      ikr::launch_tangent_gather(a->bsr(), true, true, false, a->gslice.p, a->inv_ptr.p, a->inv_idx.p, a->eblk.p, nf,
+                                 a->values(), e0, n, f->stream);
+      count(1);
+    }
   };
   if (a->tan_req && (a->tan_req != 2 || row_ok)) a->tan_path = a->tan_req;
   if (!a->tan_path) {
@@ -260,12 +265,16 @@ static void assemble_matrix_into(ikr_asm a, ikr_req r, int dbc, bool sync) {
     (a->fp32 ? f->epb_k32 : f->epb_k64) = 32;  // (these kernels have one launch shape)
     a->build_gather_map();
     const bool full = f->na > 0 || f->material != IKR_MATERIAL_NEOHOOKE;
-    a->eblk64.alloc((size_t)f->ne * (full ? 576 : ikr::kElemBlockCount * 9));
+    const int per = full ? 576 : ikr::kElemBlockCount * 9, part = a->gather_part(f->ne, sizeof(double) * per);
+    a->eblk64.alloc((size_t)part * per);
     args.blk = args.elem_mat = a->eblk64.p;
-    f->launch_elements(args, ikr::kWantK | (full ? ikr::kElemOut : ikr::kElemBlocks), false, nullptr, f->ne, 0);
-    ikr::launch_tangent_gather(a->bsr(), a->fp32, false, full, a->gslice.p, a->inv_ptr.p, a->inv_idx.p, a->eblk64.p, nf,
-                               a->values(), f->stream);
-    count(1);
+    for (int e0 = 0; e0 < f->ne; e0 += part) {
+      const int n = std::min(part, f->ne - e0);
+      f->launch_elements(args, ikr::kWantK | (full ? ikr::kElemOut : ikr::kElemBlocks), false, nullptr, n, e0);
+      ikr::launch_tangent_gather(a->bsr(), a->fp32, false, full, a->gslice.p, a->inv_ptr.p, a->inv_idx.p, a->eblk64.p,
+                                 nf, a->values(), e0, n, f->stream);
+      count(1);
+    }
   } else {
     assemble_matrix32(a, args, nf);
   }

@@ -352,12 +352,14 @@ struct ikr_asm_s {
   // slice of every block column group
   DBuf<float> eblk;
   DBuf<double> eblk64;
+  // elements whose blocks or matrices (`bytes` each) are held at a time: at most 4 GB of them
+  static int gather_part(int ne, size_t bytes) { return (int)std::min<size_t>(ne, std::max<size_t>(1, (4ull << 30) / bytes)); }
   DBuf<int32_t> inv_ptr, inv_idx, gslice;
   void build_gather_map() {
     if (inv_idx.p) return;
     ikr_fes f = fes;
     cudaStream_t s = f->stream;
-    if (64LL * f->ne >= (1LL << 31))
+    if (64LL * f->ne >= (1LL << 32))
       fail(IKR_ERR_NOT_IMPLEMENTED, "gathered tangent: too many elements for 32-bit block codes");
     DBuf<int32_t> cnt, cursor;
     cnt.alloc(npad);
