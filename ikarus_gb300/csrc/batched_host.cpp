@@ -139,57 +139,111 @@ static void plan_batch_launch(ikr_nr nr, ikr_fes f, ikr_asm a, bool fp32, const 
   }
 }
 
-// CTA groups of one launch of the one-reduction kernel (cg_halo.cu): one CTA per SM; an instance gets as many as the
-// smallest number of slices per CTA allows at which all groups fit.  False where there are more instances than SMs or a
-// CTA's share does not fit its registers and shared memory (more than 2 048 rows per CTA in FP32, 1 024 in FP64; the
-// halo is bounded by the instance, so that the launch needs no answer from the device: instances of more than about
-// 9 000 and 6 000 rows).  Instances that leave a solve only make the shares of the others smaller.
-static bool plan_halo_launch(ikr_nr nr, ikr_fes f, ikr_asm a, bool fp32, const std::vector<int>& run) {
-  auto& P = nr->plan;
-  const int n = (int)run.size(), cap = std::min(num_sms(), 160);
-  if (n > cap) return false;
-  std::vector<int> order(run);
-  auto rows = [&](int i) { return f->inst_off_h[i + 1] - f->inst_off_h[i]; };
-  auto slice_a = [&](int i) { return f->inst_off_h[i] >> 5; };
-  auto slices = [&](int i) { return ((f->inst_off_h[i + 1] - 1) >> 5) - slice_a(i) + 1; };
-  std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return rows(x) > rows(y); });
-  int lo = 1, hi = slices(order[0]) + 1;  // the slices of the instance with the most rows, one more at most
+// A launch of the one-reduction kernel (cg_halo.cu): the instances, largest first, and the slices per CTA -- one CTA per SM,
+// an instance gets as many as the smallest number of slices per CTA allows at which all groups fit.
+struct HaloWave {
+  std::vector<int> inst;
+  int q = 0;
+};
+static int inst_slices(ikr_fes f, int i) { return ((f->inst_off_h[i + 1] - 1) >> 5) - (f->inst_off_h[i] >> 5) + 1; }
+static int slices_per_cta(ikr_fes f, const int* inst, int n, int ctas) {
+  int lo = 1, hi = 1;
+  for (int k = 0; k < n; ++k) hi = std::max(hi, inst_slices(f, inst[k]));
   while (lo < hi) {
     const int q = (lo + hi) / 2;
     int64_t t = 0;
-    for (int i : run) t += (slices(i) + q - 1) / q;
-    if (t <= cap) hi = q;
+    for (int k = 0; k < n; ++k) t += (inst_slices(f, inst[k]) + q - 1) / q;
+    if (t <= ctas) hi = q;
     else lo = q + 1;
   }
-  ikr::HaloPlan S;
-  std::vector<int32_t> ci, cf, cs;
-  P.max_rows = rows(order[0]);
-  for (int i : order) {
-    const int ns = slices(i), g = (ns + lo - 1) / lo, first = (int)ci.size(), sa = slice_a(i);
+  return lo;
+}
+
+// A launch's CTA groups, and whether a CTA's share fits registers and shared memory (at most 2 048 rows per CTA in FP32, 1 024 in
+// FP64; the halo is bounded by the instance, so that the launch needs no answer from the device: instances of up to about
+// 9 000 and 6 000 rows).
+static bool split_wave(ikr_fes f, ikr_asm a, bool fp32, const HaloWave& W, ikr::HaloPlan& S, std::vector<int32_t>& ci,
+                       std::vector<int32_t>& cf, std::vector<int32_t>& cs) {
+  S = ikr::HaloPlan{};
+  ci.clear(), cf.clear(), cs.clear();
+  for (int i : W.inst) {
+    const int ns = inst_slices(f, i), g = (ns + W.q - 1) / W.q, first = (int)ci.size(), sa = f->inst_off_h[i] >> 5;
     for (int k = 0; k < g; ++k) {
       ci.push_back(i), cf.push_back(first), cs.push_back(g);
       const int s0 = sa + (int)((int64_t)k * ns / g), s1 = sa + (int)((int64_t)(k + 1) * ns / g);
       const int own = std::min(f->inst_off_h[i + 1], 32 * s1) - std::max(f->inst_off_h[i], 32 * s0);
       S.max_ns = std::max(S.max_ns, s1 - s0);
       S.max_units = std::max(S.max_units, a->slice_off_h[s1] - a->slice_off_h[s0]);
-      S.max_halo = std::max(S.max_halo, rows(i) - own);
+      S.max_halo = std::max(S.max_halo, f->inst_off_h[i + 1] - f->inst_off_h[i] - own);
     }
   }
   S.n_cta = (int)ci.size();
   S.halo_cap = S.max_halo;
-  if (!ikr::batched_halo_fits(S, fp32)) return false;
+  return ikr::batched_halo_fits(S, fp32);
+}
+
+// The instances in `run` as one launch or as two after each other, the larger instances first: an SM that holds one small
+// instance is lost to the large ones, whose share of slices sets the time of an iteration.  Measured on single systems an iteration
+// takes about 4 + 0.5 q microseconds in FP32 and 6 + 2.4 q in FP64 (q slices per CTA): the split with the smallest sum that
+// fits is taken (FP32, 128 instances: 119 -> 112 and 143 -> 132 ms per load step, 300: 353 -> 309 ms; up to 100
+// instances one launch is what this gives).  Empty where there are more than twice as many instances as SMs or none fits; `keep`: not empty, one
+// instance after the other if need be (with all SMs, an instance that fitted in a group fits).
+static std::vector<HaloWave> plan_halo(ikr_fes f, ikr_asm a, bool fp32, const std::vector<int>& run, bool keep) {
+  const int n = (int)run.size(), ctas = std::min(num_sms(), 160);
+  std::vector<int> order(run);
+  std::stable_sort(order.begin(), order.end(), [&](int x, int y) {
+    return f->inst_off_h[x + 1] - f->inst_off_h[x] > f->inst_off_h[y + 1] - f->inst_off_h[y];
+  });
+  struct Cut {
+    double t;
+    int at, qa, qb;
+  };
+  const double t0 = fp32 ? 4.0 : 6.0, t1 = fp32 ? 0.5 : 2.4;
+  std::vector<Cut> cuts;
+  if (n <= ctas) {
+    const int q = slices_per_cta(f, order.data(), n, ctas);
+    cuts.push_back({t0 + t1 * q, n, q, 0});
+  }
+  for (int k = 1; k < 8 && (cuts.empty() || cuts[0].qa > 1); ++k) {
+    const int c = n * k / 8;
+    if (c < 1 || c > ctas || n - c > ctas) continue;
+    const int x = slices_per_cta(f, order.data(), c, ctas), y = slices_per_cta(f, order.data() + c, n - c, ctas);
+    cuts.push_back({2 * t0 + t1 * (x + y), c, x, y});
+  }
+  std::stable_sort(cuts.begin(), cuts.end(), [](const Cut& x, const Cut& y) { return x.t < y.t; });
+  std::vector<HaloWave> waves;
+  ikr::HaloPlan S;
+  std::vector<int32_t> ci, cf, cs;
+  for (const Cut& c : cuts) {
+    waves.assign(1, HaloWave{std::vector<int>(order.begin(), order.begin() + c.at), c.qa});
+    if (c.at < n) waves.push_back(HaloWave{std::vector<int>(order.begin() + c.at, order.end()), c.qb});
+    bool fits = true;
+    for (const HaloWave& W : waves) fits = fits && split_wave(f, a, fp32, W, S, ci, cf, cs);
+    if (fits) return waves;
+  }
+  waves.clear();
+  for (int k = 0; keep && k < n; ++k)
+    waves.push_back(HaloWave{std::vector<int>(1, order[k]), slices_per_cta(f, &order[k], 1, ctas)});
+  return waves;
+}
+
+static void upload_wave(ikr_nr nr, ikr_fes f, ikr_asm a, bool fp32, const HaloWave& W) {
+  auto& P = nr->plan;
+  std::vector<int32_t> ci, cf, cs;
+  ikr::HaloPlan& S = P.halo_split;
+  need(split_wave(f, a, fp32, W, S, ci, cf, cs), IKR_ERR_ARG, "the batched CG's split does not fit");
+  P.max_rows = f->inst_off_h[W.inst[0] + 1] - f->inst_off_h[W.inst[0]];
   cudaStream_t s = f->stream;
+  const size_t cap = (size_t)std::min(num_sms(), 160);
   for (auto* b : {&P.cta_inst, &P.cta_first, &P.cta_size, &P.halo_cnt})
-    if (b->n < (size_t)cap) b->alloc(cap);
+    if (b->n < cap) b->alloc(cap);
   if (P.halo_rows.n < (size_t)S.n_cta * S.halo_cap) P.halo_rows.alloc((size_t)S.n_cta * S.halo_cap);
   if (P.col16.n < (size_t)a->bsr().n_padded) P.col16.alloc(a->bsr().n_padded);
   S.halo_cnt = P.halo_cnt.p, S.halo = P.halo_rows.p, S.col16 = P.col16.p;
-  P.halo_split = S;
   P.n_cta = S.n_cta;
   CK(cudaMemcpyAsync(P.cta_inst.p, ci.data(), sizeof(int32_t) * ci.size(), cudaMemcpyHostToDevice, s));
   CK(cudaMemcpyAsync(P.cta_first.p, cf.data(), sizeof(int32_t) * cf.size(), cudaMemcpyHostToDevice, s));
   CK(cudaMemcpyAsync(P.cta_size.p, cs.data(), sizeof(int32_t) * cs.size(), cudaMemcpyHostToDevice, s));
-  return true;
 }
 
 // The batched CG of one Newton iteration: the instances with act set start their PCG on -R; the solve runs as a
@@ -215,46 +269,50 @@ static void batched_cg(ikr_nr nr, ikr_fes f, ikr_asm a, const std::vector<uint8_
   int chunk = std::max(1, P.first_chunk);
   bool first = true;
   // the planner's own choice runs as the one-reduction kernel where that fits and no other solver shares the device (with
-  // more instances than SMs from the launch on at which few enough are left); the launches count as the planner's variant
+  // too many instances from the launch on at which few enough are left); the launches count as the planner's variant
   bool halo = false;
-  // it is re-planned more often than the other kernels, at most 256 iterations a launch: the CTAs of finished instances idle until the launch ends, which
-  // at six microseconds per iteration costs more than a launch (128 instances, FP32: 119 / 117 / 121 / 123 ms at most
-  // 128 / 256 / 512 / 1 024 iterations; 100 instances, FP64: 380 / 383 / 397 / 397 ms)
+  // it is re-planned more often than the other kernels, at most 256 iterations a launch: the CTAs of finished instances
+  // idle until the launch ends, which at six microseconds per iteration costs more than a launch (128 instances, FP32: 119 /
+  // 117 / 121 / 123 ms at most 128 / 256 / 512 / 1 024 iterations; 100 instances, FP64: 380 / 383 / 397 / 397 ms)
   while (!run.empty()) {
-    ikr::HaloStart start = ikr::HaloStart::kContinue;
-    if (halo) {
-      need(plan_halo_launch(nr, f, a, a->fp32, run), IKR_ERR_ARG, "the batched CG's split does not fit");
-    } else if (P.variant == -1 && P.share >= 1.0 && plan_halo_launch(nr, f, a, a->fp32, run)) {
+    std::vector<HaloWave> waves;
+    if (P.variant == -1 && P.share >= 1.0) waves = plan_halo(f, a, a->fp32, run, halo);
+    if (!waves.empty()) {
+      const ikr::HaloStart start = halo    ? ikr::HaloStart::kContinue
+                                   : first ? ikr::HaloStart::kFirst
+                                           : ikr::HaloStart::kTakeOver;
       halo = true;
-      start = first ? ikr::HaloStart::kFirst : ikr::HaloStart::kTakeOver;
-    }
-    if (halo) {
       std::vector<int> order;
       P.cur_variant = planned(nr, f, a, a->fp32, run, order).variant;
       chunk = std::min(chunk, std::max(256, P.first_chunk));
+      CK(cudaMemsetAsync(P.flag.p, 0x7f, sizeof(int32_t) * ni, s));
+      for (const HaloWave& W : waves) {
+        upload_wave(nr, f, a, a->fp32, W);
+        CK(ikr::launch_batched_halo(a->bsr(), w, P.halo_split, P.halo_cnt.p, P.halo_rows.p, P.col16.p, P.max_rows,
+                                    nr->rhs.p, nr->corr.p, f->inst_off.p, P.cta_inst.p, P.cta_first.p, P.cta_size.p,
+                                    nr->inst_rtol.p, st.linear_max_iter, chunk, start, P.st.p, nr->inst_cg_iters.p,
+                                    P.flag.p, nr->inst_cg_res.p, s));
+        count(start == ikr::HaloStart::kContinue ? 2 : 3);
+        ++P.launches;
+        ++P.launches_by_variant[P.cur_variant];
+      }
     } else {
       plan_batch_launch(nr, f, a, a->fp32, run);
+      if (P.cur_variant == 4)
+        CK(ikr::launch_batched_pcg_cluster(a->bsr(), w.minv, nr->rhs.p, nr->corr.p, P.n_cta, f->inst_off.p,
+                                           P.cta_inst.p, w.x, w.r, w.z, w.p0, w.p1, nr->inst_rtol.p,
+                                           st.linear_max_iter, chunk, first ? 1 : 0, P.st.p, nr->inst_cg_iters.p,
+                                           P.flag.p, nr->inst_cg_res.p, s));
+      else
+        CK(ikr::launch_batched_pcg(a->bsr(), a->fp32, P.cur_variant, w.minv, nr->rhs.p, nr->corr.p, P.n_cta,
+                                   f->inst_off.p, P.cta_inst.p, P.cta_first.p, P.cta_size.p, w.x, w.r, w.z, w.p0, w.p1,
+                                   w.q, nr->inst_rtol.p, st.linear_max_iter, chunk, first ? 1 : 0, P.st.p,
+                                   nr->inst_cg_iters.p, P.flag.p, nr->inst_cg_res.p, P.part.p, P.counters.p, ni,
+                                   P.cooperative, s));
+      count(1);
+      ++P.launches;
+      ++P.launches_by_variant[P.cur_variant];
     }
-    if (halo) {
-      CK(ikr::launch_batched_halo(a->bsr(), w, P.halo_split, P.halo_cnt.p, P.halo_rows.p, P.col16.p, P.max_rows,
-                                  nr->rhs.p, nr->corr.p, f->inst_off.p, P.cta_inst.p, P.cta_first.p, P.cta_size.p,
-                                  nr->inst_rtol.p, st.linear_max_iter, chunk, start, P.st.p, nr->inst_cg_iters.p,
-                                  P.flag.p, ni, nr->inst_cg_res.p, s));
-      count(start == ikr::HaloStart::kContinue ? 1 : 2);
-    } else if (P.cur_variant == 4)
-      CK(ikr::launch_batched_pcg_cluster(a->bsr(), w.minv, nr->rhs.p, nr->corr.p, P.n_cta, f->inst_off.p,
-                                         P.cta_inst.p, w.x, w.r, w.z, w.p0, w.p1, nr->inst_rtol.p, st.linear_max_iter,
-                                         chunk, first ? 1 : 0, P.st.p, nr->inst_cg_iters.p, P.flag.p,
-                                         nr->inst_cg_res.p, s));
-    else
-      CK(ikr::launch_batched_pcg(a->bsr(), a->fp32, P.cur_variant, w.minv, nr->rhs.p, nr->corr.p, P.n_cta,
-                                 f->inst_off.p, P.cta_inst.p, P.cta_first.p, P.cta_size.p, w.x, w.r, w.z, w.p0, w.p1,
-                                 w.q, nr->inst_rtol.p, st.linear_max_iter, chunk, first ? 1 : 0, P.st.p,
-                                 nr->inst_cg_iters.p, P.flag.p, nr->inst_cg_res.p, P.part.p, P.counters.p, ni,
-                                 P.cooperative, s));
-    count(1);
-    ++P.launches;
-    ++P.launches_by_variant[P.cur_variant];
     first = false;
     chunk = std::min(2 * chunk, std::max(chunk, halo ? 256 : 4096));
     P.flag.download(flag.data(), ni, s);

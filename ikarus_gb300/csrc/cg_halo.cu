@@ -795,7 +795,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1) pcg_halo_kernel(const __grid_co
         H.g.its[inst] = it;
         H.g.relres[inst] = bb > 0.0 ? sqrt(rrs / bb) : 0.0;
       }
-      atomicMin(&H.g.flag[inst], failed ? -1 : done);  // set above every flag before the launch
+      atomicMin(&H.g.flag[inst], failed ? -1 : done);  // the host sets it above every value before the launch
     }
     return;
   }
@@ -1106,7 +1106,7 @@ cudaError_t launch_batched_halo(const Bsr& A, const PcgWork& work, const HaloPla
                                 uint16_t* col16, int max_rows, const double* b, double* x_out, const int32_t* node_off,
                                 const int32_t* cta_inst, const int32_t* cta_first, const int32_t* cta_size,
                                 const double* rtol, int max_iter, int chunk, HaloStart start, double* st, int32_t* its,
-                                int32_t* flag, int n_inst, double* relres, cudaStream_t s) {
+                                int32_t* flag, double* relres, cudaStream_t s) {
   const Layout L = work.fp32 ? layout_of<float>(P, warps_of(true, 0)) : layout_of<double>(P, warps_of(false, 0));
   if (!L.ok) return cudaErrorInvalidConfiguration;
   PcgWork w = work;
@@ -1115,7 +1115,6 @@ cudaError_t launch_batched_halo(const Bsr& A, const PcgWork& work, const HaloPla
   w.keep_g = groups < kept ? groups : kept;
   const HaloGroups g{cta_inst, cta_first, cta_size, node_off, rtol, max_iter, chunk, w.p0, st, its, flag, relres, x_out};
   cudaError_t e = cudaMemsetAsync(w.part_c, 0, sizeof(double) * kHaloWords, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(flag, 0x7f, sizeof(int32_t) * n_inst, s);
   if (e != cudaSuccess) return e;
   halo_plan_kernel<true><<<P.n_cta, 1024, (max_rows + 31) / 32 * 8, s>>>(A, P, g, nullptr, cnt, halo, col16);
   if (start == HaloStart::kTakeOver && w.fp32)

@@ -346,14 +346,14 @@ cudaError_t launch_batched_pcg(const Bsr& A, bool fp32, int variant, const void*
 // touch split evenly over its group.  P: n_cta, chunk 32, the cap of the halo lists and the largest halo, slices and block
 // columns of a CTA (bounds that the host knows); cnt (n_cta), halo (n_cta x halo_cap) and col16 (n_padded) are filled
 // by the launch, which also needs the rows of the largest instance.  st holds b.b between the launches, w.p0 holds p, and
-// w.p1 the published rows.  A solve may go over from the kernels above to this one (kTakeOver), not back.
+// w.p1 the published rows; flag holds a value above every status before the launch.  A solve may go over from the kernels above to this one (kTakeOver), not back.
 enum class HaloStart { kFirst, kTakeOver, kContinue };
 bool batched_halo_fits(const HaloPlan& P, bool fp32);
 cudaError_t launch_batched_halo(const Bsr& A, const PcgWork& w, const HaloPlan& P, int32_t* cnt, int32_t* halo,
                                 uint16_t* col16, int max_rows, const double* b, double* x_out, const int32_t* node_off,
                                 const int32_t* cta_inst, const int32_t* cta_first, const int32_t* cta_size,
                                 const double* rtol, int max_iter, int chunk, HaloStart start, double* st, int32_t* its,
-                                int32_t* flag, int n_inst, double* relres, cudaStream_t s);
+                                int32_t* flag, double* relres, cudaStream_t s);
 // FP32 only: one instance per cluster of 16 CTAs (cluster_inst per cluster), at most batched_cluster_rows() rows and
 // batched_cluster_width() blocks per row; vectors and sums through distributed shared memory; same state protocol
 // (st, its, flag, x_out).  capacity: clusters co-resident on the device (more run in waves; clusters never wait on
