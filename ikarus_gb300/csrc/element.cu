@@ -1103,7 +1103,8 @@ __global__ void __launch_bounds__(256) tangent_gather_kernel(Bsr A, const int32_
   }
   uint8_t fr = 0, fc = 0;
   const int col = A.col_sell[b];
-  if (nf && c1 > c0) fr = nf[row], fc = nf[col];
+  // a node without elements has no pattern entry; the first padded block of its row stands for the diagonal
+  if (nf && (c1 > c0 || (row < A.n_rows && A.diag[row] == b))) fr = nf[row], fc = nf[col];
 #pragma unroll
   for (int i = 0; i < 3; ++i)
 #pragma unroll
