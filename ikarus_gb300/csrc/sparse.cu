@@ -131,7 +131,7 @@ __device__ __forceinline__ int32_t block_id(const int32_t* __restrict__ slice_of
 __global__ void slice_len_kernel(const int32_t* __restrict__ row_ptr, int nn, int32_t* slice_len) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= (nn + 31) / 32) return;
-  int m = 0;
+  int m = 1;  // rows without elements have a padded block for their diagonal, whole slices of them too
   for (int r = 32 * s; r < min(nn, 32 * s + 32); ++r) m = max(m, row_ptr[r + 1] - row_ptr[r]);
   slice_len[s] = m;
 }

@@ -1,5 +1,5 @@
-"""Clamped nodes that no element uses: their rows of the tangent are the identity (Full Dirichlet treatment), so the
-systems around them are solved as without them."""
+"""Clamped nodes that no element uses: their rows of the tangent are the identity (Full Dirichlet treatment) wherever they
+sit in the slices of 32 rows, so the systems around them are solved as without them."""
 import numpy as np
 import pytest
 import scipy.sparse.linalg as spla
@@ -8,8 +8,9 @@ from ikarus_gb300 import problems
 
 pytestmark = pytest.mark.gpu
 
-# 36 nodes of the mesh take a slice of 32 rows and four of the next: unused nodes in front of and behind them
-PLACES = {"same_slice": (0, 3), "in_front": (5, 0)}
+# 36 nodes of the mesh take a slice and four rows: unused nodes in the second slice, two slices of them behind, one slice
+# and one row in front
+PLACES = {"same_slice": (0, 3), "slices_behind": (0, 70), "slices_in_front": (33, 0)}
 
 
 def _padded(p, front, behind):
