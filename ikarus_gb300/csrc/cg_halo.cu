@@ -146,17 +146,43 @@ __device__ __noinline__ Num warp_sum(long long m, int x) {
   const int k = __clzll(S < 0 ? ~S : S) - 3;  // the highest bit goes to bit 60
   return {k >= 0 ? S << k : S >> 1, X - (k >= 0 ? k : -1)};
 }
-// Warp sums of three values at once (the redux chains overlap), as S * 2^x with |S| < 2^62, to slot `warp` of the CTA's
-// lists S[k * stride], x[k * stride]
-// (PAIR: the second value is v1 + v2, v2 below a unit in the last place of v1, and there is no third)
-template <typename T, bool PAIR = false>
-__device__ __noinline__ void warp_parts(T v0, T v1, T v2, long long* S, int* x, int stride) {
-  __syncwarp();
-  Num u[3] = {num_of(v0), num_of(v1), num_of(v2)};
-  if (PAIR) {
-    u[1].S += shift_right(u[2].S, u[1].x - u[2].x);
-    u[2] = {0, kZeroExp};
+// S / 16 * 2^x, |S| < 2^58: what the warp sums take
+struct Num16 {
+  long long S;
+  int x;
+};
+template <typename T>
+__device__ __forceinline__ Num16 num16_of(T v) {
+  const Num u = num_of(v);
+  return {u.S * 16, u.x};
+}
+__device__ __forceinline__ Num16 num16_of(Num16 v) { return v; }
+// Exact squares of floats, summed to 56 bits of the largest: at most 16 squares of 48 bits, ten bits up.  (Two floats, the
+// square and its rounding error, underflow below 1e-19 and have 48 bits; a conversion and an addition in FP64 per square
+// load GB300's narrow FP64 pipe.)
+struct SquareSum {
+  long long S = 0;
+  int x = kZeroExp;
+  __device__ __forceinline__ void add(float v) {
+    const uint32_t b = __float_as_uint(v);
+    const int e = (int)((b >> 23) & 255u);
+    const uint32_t f = (b & 0x7fffffu) | (e ? 1u << 23 : 0u);
+    const int xv = e == 255 ? kBadExp : f == 0 ? kZeroExp : 2 * (e ? e : 1) - 310, X = x > xv ? x : xv;
+    S = shift_right(S, X - x) + shift_right((long long)((uint64_t)f * f << 10), X - xv);
+    x = X;
   }
+  __device__ __forceinline__ Num16 num16() const {
+    if (x == kBadExp || S == 0) return {0, x};
+    const int k = __clzll(S) - 6;  // the highest bit goes to bit 57
+    return {k >= 0 ? S << k : S >> -k, x + 4 - k};
+  }
+};
+// Warp sums of three values at once (the redux chains overlap), as S * 2^x with |S| < 2^62, to slot `warp` of the CTA's
+// lists S[k * stride], x[k * stride].  The second may be a SquareSum's.
+template <typename T, typename U>
+__device__ __noinline__ void warp_parts(T v0, U v1, T v2, long long* S, int* x, int stride) {
+  __syncwarp();
+  const Num16 u[3] = {num16_of(v0), num16_of(v1), num16_of(v2)};
   int X[3];
   uint32_t lo[3], mid[3];
   int hi[3];
@@ -164,7 +190,7 @@ __device__ __noinline__ void warp_parts(T v0, T v1, T v2, long long* S, int* x, 
   for (int k = 0; k < 3; ++k) X[k] = __reduce_max_sync(0xffffffffu, u[k].x);
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    const long long a = shift_right(u[k].S * 16, X[k] - u[k].x);
+    const long long a = shift_right(u[k].S, X[k] - u[k].x);
     lo[k] = __reduce_add_sync(0xffffffffu, (uint32_t)a & 0x7ffffffu);
     mid[k] = __reduce_add_sync(0xffffffffu, (uint32_t)(a >> 27) & 0x7ffffffu);
     hi[k] = __reduce_add_sync(0xffffffffu, (int)(a >> 54));
@@ -520,29 +546,22 @@ __global__ void __launch_bounds__(WARPS * 32, 1) pcg_halo_kernel(const __grid_co
       if (!STREAM && ((pend >> j) & 1u)) got[j] = fetch_row(H.p, hl[tid + j * kThreads], tag, vx[j], vy[j], vz[j]);
     }
     if (warp < nwr) {
-      // GROUPS in FP32: r.r as a pair of floats, exact squares and compensated sums (the instances' tolerances go down to
-      // where 24 bits of a lane's squares would show)
-      constexpr bool kPair = GROUPS && sizeof(T) == 4;
-      T srz = T(0), srr = T(0), low = T(0);
+      // GROUPS in FP32: r.r of exact squares, to more than FP64's bits and in a wider range than FP32's (the instances'
+      // tolerances go down to where 24 bits of a lane's squares would show)
+      constexpr bool kExact = GROUPS && sizeof(T) == 4;
+      static_assert(MAXP * NC <= 16, "squares of a lane");
+      T srz = T(0), srr = T(0);
+      SquareSum sq;
 #pragma unroll
       for (int j = 0; j < MAXP; ++j)  // zero where the lane owns nothing
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
           srz += rr[j][c] * zr[j][c];
-          if constexpr (kPair) {
-            const T v = rr[j][c], sq = v * v, t = srr + sq, d = t - srr;
-            low += fma(v, v, -sq) + ((srr - (t - d)) + (sq - d));
-            srr = t;
-          } else {
-            srr += rr[j][c] * rr[j][c];
-          }
+          if constexpr (kExact) sq.add(rr[j][c]);
+          else srr += rr[j][c] * rr[j][c];
         }
-      if constexpr (kPair) {
-        const T t = srr + low;
-        low -= t - srr;
-        srr = t;
-      }
-      warp_parts<T, kPair>(srz, srr, low, &swS[3][warp], &swx[3][warp], WARPS);
+      if constexpr (kExact) warp_parts<T>(srz, sq.num16(), T(0), &swS[3][warp], &swx[3][warp], WARPS);
+      else warp_parts<T>(srz, srr, T(0), &swS[3][warp], &swx[3][warp], WARPS);
     }
 #pragma unroll
     for (int j = 0; j < kBatch; ++j)
