@@ -9,7 +9,7 @@
 //   * data carries its own arrival: a published row of p, and each published CTA sum, is a 128-bit word with the
 //     iteration number inside, written and polled as one access.  No fence, no counter, no second read;
 //   * an iteration has one reduction.  q = K p and w = M^-1 q give p.q, z.q, q.w, r.z and r.r together; then
-//       alpha = rz / pq,  r'z' = rz - 2 alpha zq + alpha^2 qw,  beta = r'z' / rz
+//       alpha = rz / pq,  r'z' = rz - 2 alpha zq + alpha^2 qw,  beta = r'z' / rz       (alpha rounded as it is used)
 //     (r.z and r.r are formed from the vectors in every iteration, so nothing drifts; r, z, p and x follow the same
 //     recurrences as the other forms).  r.r tells of the previous update: a solve ends one product later;
 //   * the blocks of a CTA are contiguous in the sliced-ELL values; its warps take equal runs of block columns whatever
@@ -214,24 +214,6 @@ __device__ __forceinline__ double to_double(const Num& u) {
   return __longlong_as_double((b & 0x800fffffffffffffll) | ((long long)e << 52));
 }
 
-// 1 / d by Newton's iteration y <- y + y (1 - d y) from a single-precision reciprocal of the leading bits: 46 bits after
-// one step, which a result rounded to FP32 needs, all but the last after two.  d is finite with an exponent far from
-// the ends of the range.  Half the FP64 instructions of the general division, each of which takes about 60 cycles.
-template <typename T>
-__device__ __forceinline__ double reciprocal(double d) {
-  const uint32_t hi = (uint32_t)(__double_as_longlong(d) >> 32), lo = (uint32_t)__double_as_longlong(d);
-  const float m = __uint_as_float(0x3f800000u | ((hi & 0xfffffu) << 3) | (lo >> 29));  // [1, 2)
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(m));
-  const uint32_t rb = __float_as_uint(r);  // (0.5, 1]
-  // r's exponent less that of d, in the double's bias
-  const uint32_t e = (rb >> 23) + 1023u - 127u + 1023u - ((hi >> 20) & 2047u);
-  double y = __longlong_as_double((long long)pack32(rb << 29, (hi & 0x80000000u) | (e << 20) | ((rb & 0x7fffffu) >> 3)));
-  y = fma(y, fma(-d, y, 1.0), y);
-  if (sizeof(T) == 8) y = fma(y, fma(-d, y, 1.0), y);
-  return y;
-}
-
 // Independent instances of one element set, a group of CTAs each (the GROUPS form of the kernel): CTA b is number
 // b - first[b] of the size[b] that serve instance inst[b], whose rows are [node_off[inst], node_off[inst + 1]).  The slices
 // an instance's rows touch are split evenly over its group; lanes of other instances' rows compute along unseen.
@@ -296,7 +278,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1) pcg_halo_kernel(const __grid_co
   __shared__ __align__(8) uint64_t bars[WARPS][STREAM ? kMaxRing : 1];
   __shared__ long long swS[kSums + 1][WARPS];  // the warps' sums
   __shared__ int swx[kSums + 1][WARPS];
-  __shared__ double ssum[kSums];
+  __shared__ double ssum[kSums], srec[2];  // the grid's sums; 1 / p.q and 1 / r.z
   __shared__ T s_ab[2];
   __shared__ int s_done;
   __shared__ int s_fail;
@@ -722,12 +704,18 @@ __global__ void __launch_bounds__(WARPS * 32, 1) pcg_halo_kernel(const __grid_co
 #pragma unroll
       for (int j = 0; j < kMaxCtas / 32; ++j) a += shift_right(t[j].S >> 6, X - t[j].x);
       const Num g = warp_sum(a, X == kBadExp ? kBadExp : X + 6);
-      if (lane == 0) ssum[warp] = to_double(g);
+      if (lane == 0) {
+        const double v = to_double(g);
+        ssum[warp] = v;
+        if (warp == 0) srec[0] = 1.0 / v;
+        if (warp == 3) srec[1] = 1.0 / v;  // off the critical path: r.z is here before p.q
+      }
       asm volatile("bar.sync 1, %0;" ::"n"(kSums * 32) : "memory");
       if (tid == 0) {
-        double pq = ssum[0], zq = ssum[1], qw = ssum[2];
-        const int ex = (int)((__double_as_longlong(pq) >> 52) & 2047);
-        double num = rz = ssum[3];
+        const double pq = ssum[0], zq = ssum[1], qw = ssum[2];
+        auto exponent = [](double v) { return (int)((__double_as_longlong(v) >> 52) & 2047); };
+        const int ex = exponent(pq);
+        rz = ssum[3];
         rrs = ssum[4];
         int d = 0;
         double alpha = 0.0;
@@ -735,17 +723,16 @@ __global__ void __launch_bounds__(WARPS * 32, 1) pcg_halo_kernel(const __grid_co
         if ((GROUPS || it > 0) && __double_as_longlong(rrs) <= __double_as_longlong(tol2)) d = 1;
         else if ((GROUPS || it > 0) && it >= maxit) d = GROUPS ? 1 : 2;
         else if ((__double_as_longlong(pq) << 1) == 0 || ex == 2047) d = GROUPS ? 2 : 3;  // negative curvature alone does not stop CG
-        else {
-          // alpha = rz / pq and beta = (rz - 2 alpha zq + alpha^2 qw) / rz = 1 + (alpha qw - 2 zq) / pq from one
-          // reciprocal; sums whose p.q is near the ends of the range are scaled by a power of two
-          if (ex < 64 || ex > 1980) {
-            const double f = ex < 64 ? 0x1p200 : 0x1p-200;
-            pq *= f, zq *= f, qw *= f, num *= f;
-          }
-          const double ip = reciprocal<T>(pq);
-          alpha = num * ip;
-          beta = fma(ip, fma(alpha, qw, -2.0 * zq), 1.0);
-          if (sizeof(T) == 8) alpha = fma(fma(-alpha, pq, num), ip, alpha);
+        else if (const int ez = exponent(rz); ex >= 64 && ex <= 1980 && ez >= 64 && ez <= 1980) {
+          // beta for the alpha that the vectors are updated with: rounded to FP32 it is off by more than the sums are.  In
+          // FP64 alpha's last bit is corrected beside it
+          alpha = rz * srec[0];
+          const double a = double(T(alpha));
+          beta = fma(a * srec[1], fma(a, qw, -2.0 * zq), 1.0);
+          if (sizeof(T) == 8) alpha = fma(fma(-alpha, pq, rz), srec[0], alpha);
+        } else {  // sums near the ends of the range
+          alpha = rz / pq;
+          beta = 1.0 + (double(T(alpha)) * qw - 2.0 * zq) / pq;
         }
         s_ab[0] = T(alpha);
         s_ab[1] = T(beta);
