@@ -263,6 +263,7 @@ SIGNATURES = {
     "ikr_linear_solver_coarse_info": ([_vp, _ip], C.c_int),
     "ikr_linear_solver_set_coarse_refresh": ([_vp, _I], C.c_int),
     "ikr_assembler_set_tangent_kernel": ([_vp, _I], C.c_int),
+    "ikr_assembler_set_gather_part": ([_vp, C.c_int64], C.c_int),
     "ikr_assembler_tangent_kernel": ([_vp, _ip], C.c_int),
     "ikr_linear_solver_solve2": ([_vp, _vp, _dp, _dp, _dp, _dp], C.c_int),
     "ikr_path_following_create": ([C.POINTER(_vp), _vp, _I, _D, _I, _I, _ip], C.c_int),
@@ -820,6 +821,11 @@ class SparseFlatAssembler:
         """FP32 displacement-based tangent: 1 coloured element kernel, 2 row kernel, 3 element blocks + gather, 0 timed
         choice."""
         _err(lib().ikr_assembler_set_tangent_kernel(self.h, int(path)))
+
+    def set_gather_part(self, n_elems=0):
+        """Gathered tangents hold the blocks or matrices of at most n_elems elements at a time (0: 4 GB of them); the
+        tangent does not depend on it."""
+        _err(lib().ikr_assembler_set_gather_part(self.h, int(n_elems)))
 
     def tangent_kernel(self):
         """The FP32 tangent kernel in use (0 = not chosen yet, 1 coloured, 2 rows)."""

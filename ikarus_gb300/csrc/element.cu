@@ -1053,14 +1053,16 @@ __global__ void tangent_inv_sort_kernel(const uint32_t* __restrict__ ptr, uint32
 // One thread per padded block: the sum of its element blocks in ascending order, the Full Dirichlet treatment, and
 // the nine entries written to the entry-interleaved slice (a warp writes 9 x 32 contiguous values).  The elements' blocks
 // come as the 36 distinct ones of an element, or (FULL) as column-major 24 x 24 matrices.  Sums in S (the type of the
-// element blocks), rounded to T once.
-template <typename T, typename S, bool FULL>
+// element blocks), rounded to T once.  PART: the elements [e0, e0 + n) of a set that is gathered in parts, ascending; the
+// sums over the parts before are in `sums` (which may be val where the types are the same), and only the last part
+// writes the matrix.
+template <typename T, typename S, bool FULL, bool PART>
 __global__ void __launch_bounds__(256) tangent_gather_kernel(Bsr A, const int32_t* __restrict__ gslice,
                                                              const uint32_t* __restrict__ ptr,
                                                              const uint32_t* __restrict__ inv,
                                                              const S* __restrict__ blk,
-                                                             const uint8_t* __restrict__ nf, T* __restrict__ val,
-                                                             int e0, int n) {
+                                                             const uint8_t* __restrict__ nf, T* val, S* sums, int e0,
+                                                             int n, bool last) {
   const int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (b >= A.n_padded) return;
   const int g = (int)(b >> 5), l = (int)(b & 31);
@@ -1070,14 +1072,15 @@ __global__ void __launch_bounds__(256) tangent_gather_kernel(Bsr A, const int32_
   for (int k = 0; k < 9; ++k) acc[k] = S(0);
   const uint32_t c0 = ptr[b], c1 = ptr[b + 1];
   T* out = val + (size_t)g * 288 + l;
-  if (e0 > 0) {  // a later part of the elements: on top of the former parts' sums
+  S* sum = sums + (size_t)g * 288 + l;
+  if (PART && e0 > 0) {
 #pragma unroll
-    for (int k = 0; k < 9; ++k) acc[k] = S(out[32 * k]);
+    for (int k = 0; k < 9; ++k) acc[k] = sum[32 * k];
   }
   for (uint32_t c = c0; c < c1; ++c) {
     const uint32_t code = __ldg(inv + c);
-    const int e = (int)(code >> 6) - e0, I = (code >> 3) & 7, J = code & 7;
-    if ((unsigned)e >= (unsigned)n) continue;
+    const int e = (int)(code >> 6) - (PART ? e0 : 0), I = (code >> 3) & 7, J = code & 7;
+    if (PART && (unsigned)e >= (unsigned)n) continue;
     S v[9];
     if constexpr (FULL) {
       const S* src = blk + (size_t)e * 576 + 72 * J + 3 * I;
@@ -1100,6 +1103,11 @@ __global__ void __launch_bounds__(256) tangent_gather_kernel(Bsr A, const int32_
         for (int k = 0; k < 9; ++k) acc[k] += v[k];
       }
     }
+  }
+  if (PART && !last) {
+#pragma unroll
+    for (int k = 0; k < 9; ++k) sum[32 * k] = acc[k];
+    return;
   }
   uint8_t fr = 0, fc = 0;
   const int col = A.col_sell[b];
@@ -1211,18 +1219,21 @@ void launch_tangent_inverse_fill(const int32_t* slot, int n_elems, const int32_t
 }
 template <typename T, typename S, bool FULL>
 static void gather_t(const Bsr& A, const int32_t* gslice, const int32_t* inv_ptr, const int32_t* inv, const void* blk,
-                     const uint8_t* nf, void* val, int e0, int n, cudaStream_t s) {
-  tangent_gather_kernel<T, S, FULL><<<(unsigned)((A.n_padded + 255) / 256), 256, 0, s>>>(
-      A, gslice, (const uint32_t*)inv_ptr, (const uint32_t*)inv, (const S*)blk, nf, (T*)val, e0, n);
+                     const uint8_t* nf, void* val, void* sums, int e0, int n, int n_elems, cudaStream_t s) {
+  const bool last = e0 + n >= n_elems;
+  auto kern = e0 == 0 && last ? tangent_gather_kernel<T, S, FULL, false> : tangent_gather_kernel<T, S, FULL, true>;
+  kern<<<(unsigned)((A.n_padded + 255) / 256), 256, 0, s>>>(A, gslice, (const uint32_t*)inv_ptr, (const uint32_t*)inv,
+                                                            (const S*)blk, nf, (T*)val, (S*)sums, e0, n, last);
 }
 void launch_tangent_gather(const Bsr& A, bool fp32_val, bool fp32_blk, bool full, const int32_t* gslice,
                            const int32_t* inv_ptr, const int32_t* inv, const void* blk, const uint8_t* node_fixed,
-                           void* val, int e0, int n, cudaStream_t s) {
+                           void* val, void* sums, int e0, int n, int n_elems, cudaStream_t s) {
   if (A.n_padded <= 0) return;
-  if (fp32_blk) gather_t<float, float, false>(A, gslice, inv_ptr, inv, blk, node_fixed, val, e0, n, s);
-  else if (full && fp32_val) gather_t<float, double, true>(A, gslice, inv_ptr, inv, blk, node_fixed, val, e0, n, s);
-  else if (full) gather_t<double, double, true>(A, gslice, inv_ptr, inv, blk, node_fixed, val, e0, n, s);
-  else gather_t<double, double, false>(A, gslice, inv_ptr, inv, blk, node_fixed, val, e0, n, s);
+  auto launch = fp32_blk           ? gather_t<float, float, false>
+                : full && fp32_val ? gather_t<float, double, true>
+                : full             ? gather_t<double, double, true>
+                                   : gather_t<double, double, false>;
+  launch(A, gslice, inv_ptr, inv, blk, node_fixed, val, sums, e0, n, n_elems, s);
 }
 void launch_node_corners(const int32_t* conn, int n_elems, int n_nodes, const int32_t* ptr, int32_t* codes,
                          cudaStream_t s) {

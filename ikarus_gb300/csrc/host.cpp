@@ -198,7 +198,7 @@ static void assemble_matrix32(ikr_asm a, ikr::ElemArgs& args, const uint8_t* nf)
       const int n = std::min(part, f->ne - e0);
       f->launch_elements(t, ikr::kWantK | ikr::kElemBlocks, true, nullptr, n, e0);
       ikr::launch_tangent_gather(a->bsr(), true, true, false, a->gslice.p, a->inv_ptr.p, a->inv_idx.p, a->eblk.p, nf,
-                                 a->values(), e0, n, f->stream);
+                                 a->values(), a->values(), e0, n, f->ne, f->stream);
       count(1);
     }
   };
@@ -268,11 +268,16 @@ static void assemble_matrix_into(ikr_asm a, ikr_req r, int dbc, bool sync) {
     const int per = full ? 576 : ikr::kElemBlockCount * 9, part = a->gather_part(f->ne, sizeof(double) * per);
     a->eblk64.alloc((size_t)part * per);
     args.blk = args.elem_mat = a->eblk64.p;
+    void* sums = a->values();
+    if (a->fp32 && part < f->ne) {  // FP64 sums over the parts, rounded with the last
+      a->gsum.alloc(9 * (size_t)a->npad);
+      sums = a->gsum.p;
+    }
     for (int e0 = 0; e0 < f->ne; e0 += part) {
       const int n = std::min(part, f->ne - e0);
       f->launch_elements(args, ikr::kWantK | (full ? ikr::kElemOut : ikr::kElemBlocks), false, nullptr, n, e0);
       ikr::launch_tangent_gather(a->bsr(), a->fp32, false, full, a->gslice.p, a->inv_ptr.p, a->inv_idx.p, a->eblk64.p,
-                                 nf, a->values(), e0, n, f->stream);
+                                 nf, a->values(), sums, e0, n, f->ne, f->stream);
       count(1);
     }
   } else {
@@ -1142,6 +1147,12 @@ int ikr_assembler_set_tangent_kernel(ikr_asm a, int32_t path) {
          "tangent kernel: 0 timed choice, 1 coloured, 2 rows, 3 element blocks + gather");
     a->tan_req = path;
     a->tan_path = path;
+  });
+}
+int ikr_assembler_set_gather_part(ikr_asm a, int64_t n_elems) {
+  return guarded([&] {
+    need(a && n_elems >= 0, IKR_ERR_ARG, "gathered tangents: elements at a time, 0 for the default");
+    a->part_req = n_elems;
   });
 }
 int ikr_assembler_tangent_kernel(ikr_asm a, int32_t* path) {

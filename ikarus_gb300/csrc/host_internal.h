@@ -351,9 +351,12 @@ struct ikr_asm_s {
   // gathered assembly: the blocks (FP32, FP64) or FP64 matrices of every element, the inverse element-to-block map, the
   // slice of every block column group
   DBuf<float> eblk;
-  DBuf<double> eblk64;
-  // elements whose blocks or matrices (`bytes` each) are held at a time: at most 4 GB of them
-  static int gather_part(int ne, size_t bytes) { return (int)std::min<size_t>(ne, std::max<size_t>(1, (4ull << 30) / bytes)); }
+  DBuf<double> eblk64, gsum;
+  // elements whose blocks or matrices (`bytes` each) are held at a time: at most 4 GB of them, or as asked for
+  int64_t part_req = 0;
+  int gather_part(int ne, size_t bytes) const {
+    return (int)std::min<size_t>(ne, part_req > 0 ? (size_t)part_req : std::max<size_t>(1, (4ull << 30) / bytes));
+  }
   DBuf<int32_t> inv_ptr, inv_idx, gslice;
   void build_gather_map() {
     if (inv_idx.p) return;

@@ -123,14 +123,15 @@ constexpr int kElemBlockCount = 36;
 // gathered tangent assembly (element.cu): inverse of the element-to-block map -- for every padded block id the element
 // blocks that add to it, e * 64 + 8 I + J for the corner pair (I, J), ascending -- and the gather that sums them, applies
 // the Full Dirichlet treatment (node_fixed; unit diagonal) and writes every entry of every slice once.  blk: the 36
-// distinct blocks (FP32 or FP64), or with `full` the FP64 24 x 24 column-major matrices, of elements [e0, e0 + n); with e0 > 0
-// they are added to the sums of the elements before.  The map's codes and offsets are unsigned.
+// distinct blocks (FP32 or FP64), or with `full` the FP64 24 x 24 column-major matrices, of elements [e0, e0 + n) of n_elems:
+// parts in ascending order, the sums of the parts before in `sums` (values in the blocks' type, val itself where that is the
+// type), the matrix written with the last part.  The map's codes and offsets are unsigned.
 void launch_tangent_inverse_count(const int32_t* slot, int n_elems, int32_t* cnt, cudaStream_t s);
 void launch_tangent_inverse_fill(const int32_t* slot, int n_elems, const int32_t* ptr, int32_t* cursor, int32_t* inv,
                                  int64_t n_padded, cudaStream_t s);
 void launch_tangent_gather(const Bsr& A, bool fp32_val, bool fp32_blk, bool full, const int32_t* gslice,
                            const int32_t* inv_ptr, const int32_t* inv, const void* blk, const uint8_t* node_fixed,
-                           void* val, int e0, int n, cudaStream_t s);
+                           void* val, void* sums, int e0, int n, int n_elems, cudaStream_t s);
 // gathered residual assembly: the elements of every node (ascending, from launch_node_elem_fill) as 8 e + corner, and R
 // of every dof as the sum of its elements' forces vec (24 per element), zero where node_fixed says so
 void launch_node_corners(const int32_t* conn, int n_elems, int n_nodes, const int32_t* ptr, int32_t* codes,

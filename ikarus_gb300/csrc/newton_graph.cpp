@@ -41,7 +41,7 @@ std::vector<const void*> graph_key(ikr_nr nr, ikr_req r) {
           w.part_a, w.part_b, v(w.spmv_kind), v(w.keep_g), v(w.grid), v(w.barrier_polls), v(f->epb_r),
           v(a->fp32 ? f->epb_k32 : f->epb_k64), v(a->tan_path), a->me_idx.p, v((int64_t)a->me_idx.n), a->pl_dof.p,
           v((int64_t)a->pl_dof.n), f->trac.p, f->trac_idx.p, f->args().ext, v(nr->st.linear_max_iter),
-          v(ls->point_jacobi), a->eblk.p, a->eblk64.p, f->fel.p,
+          v(ls->point_jacobi), a->eblk.p, a->eblk64.p, v(a->part_req), f->fel.p,
           v((int64_t)ls->ho.made)};
 }
 

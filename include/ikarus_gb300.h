@@ -292,6 +292,9 @@ int ikr_cg_kind_ranges(int32_t* out4);
  * the same FP32 tangent up to the order of the FP32 additions. */
 int ikr_assembler_set_tangent_kernel(ikr_asm a, int32_t path);
 int ikr_assembler_tangent_kernel(ikr_asm a, int32_t* path);
+/* no reference counterpart, for tests: gathered tangents (FP64 and EAS ones, kernel 3 of the FP32 ones) hold the blocks or
+ * matrices of at most this many elements at a time; 0 (default): 4 GB of them.  The tangent does not depend on it. */
+int ikr_assembler_set_gather_part(ikr_asm a, int64_t n_elems);
 /* no reference counterpart: solves with two right-hand sides and one tangent (path following's bordered
  * system) run both CGs in one persistent launch that streams the matrix once per iteration (on = 1, default)
  * or one after the other (0) */
