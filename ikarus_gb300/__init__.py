@@ -177,6 +177,7 @@ SIGNATURES = {
     "ikr_newton_set_batched_cg": ([_vp, _I, _I], C.c_int),
     "ikr_newton_batched_cg_launches": ([_vp, _i64p], C.c_int),
     "ikr_newton_batched_cg_variant_launches": ([_vp, _i64p], C.c_int),
+    "ikr_newton_batched_cg_group_launches": ([_vp, _i64p], C.c_int),
     "ikr_batched_plan_preview": ([_I, _ip, _ip, _I, _I, _ip, _I, _ip, _ip], C.c_int),
     "ikr_newton_set_batched_take_out": ([_vp, _I], C.c_int),
     "ikr_load_control_set_escalation": ([_vp, _vp, _vp], C.c_int),
@@ -1291,9 +1292,17 @@ class NewtonRaphson:
         _err(lib().ikr_newton_set_batched_take_out(self.h, int(bool(unsolved_linear))))
 
     def batched_cg_variant_launches(self):
-        """Batched CG launches since creation per kernel variant 0..5."""
+        """Batched CG launches since creation per kernel variant 0..5; groups of the one-reduction CG count under the
+        variant that the planner would have taken."""
         out = np.zeros(6, dtype=np.int64)
         _err(lib().ikr_newton_batched_cg_variant_launches(self.h, _ptr(out, C.c_int64)))
+        return out
+
+    def batched_cg_group_launches(self):
+        """Batched CG launches that ran as groups of the one-reduction CG: (solves started, taken over from the planner's
+        kernels, continued)."""
+        out = np.zeros(3, dtype=np.int64)
+        _err(lib().ikr_newton_batched_cg_group_launches(self.h, _ptr(out, C.c_int64)))
         return out
 
     def batched_cg_launches(self):

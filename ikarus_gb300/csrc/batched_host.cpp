@@ -295,6 +295,7 @@ static void batched_cg(ikr_nr nr, ikr_fes f, ikr_asm a, const std::vector<uint8_
         count(start == ikr::HaloStart::kContinue ? 2 : 3);
         ++P.launches;
         ++P.launches_by_variant[P.cur_variant];
+        ++P.group_launches[(int)start];
       }
     } else {
       plan_batch_launch(nr, f, a, a->fp32, run);

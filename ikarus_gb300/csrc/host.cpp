@@ -1495,6 +1495,12 @@ int ikr_newton_batched_cg_variant_launches(ikr_nr nr, int64_t* by_variant6) {
     for (int v = 0; v < 6; ++v) by_variant6[v] = nr->plan.launches_by_variant[v];
   });
 }
+int ikr_newton_batched_cg_group_launches(ikr_nr nr, int64_t* by_start3) {
+  return guarded([&] {
+    need(nr && by_start3, IKR_ERR_ARG, "null argument");
+    for (int k = 0; k < 3; ++k) by_start3[k] = nr->plan.group_launches[k];
+  });
+}
 int ikr_newton_set_batched_take_out(ikr_nr nr, int32_t unsolved_linear) {
   return guarded([&] {
     need(nr, IKR_ERR_ARG, "null argument");

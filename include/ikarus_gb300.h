@@ -497,6 +497,9 @@ int ikr_newton_set_batched_cg(ikr_nr nr, int32_t variant, int32_t first_chunk);
 int ikr_newton_batched_cg_launches(ikr_nr nr, int64_t* n);
 /* the same per kernel variant 0..5 (six values) */
 int ikr_newton_batched_cg_variant_launches(ikr_nr nr, int64_t* by_variant6);
+/* those of them that ran as groups of the one-reduction CG: solves started, solves taken over from the planner's kernels,
+ * solves continued (three values) */
+int ikr_newton_batched_cg_group_launches(ikr_nr nr, int64_t* by_start3);
 /* the batched CG's planner on given capacities, without a device (tests): n running instances with their rows and
  * widest slice (blocks), the precision, a forced variant (-1: the planner's choice), the co-resident CTAs of each
  * variant 0..5 (caps6; entry 4 unused) and the co-resident 16-CTA clusters; gives the variant and the CTAs per
