@@ -993,8 +993,6 @@ def run_path_following(args):
            "unit": "s", "higher_is_better": False,
            "config": {"workload": "cantilever_128x32x32_jittered", "elements": p.mesh.n_elems, "dofs": p.n_dofs,
                       "path_following": "ArcLength, AdaptiveStepSizing::NoOp", "steps": steps,
-                      "bordered_solve": "two CG columns one after the other" if args.no_multi_rhs else
-                                        "two CG columns in one persistent launch (one matrix stream per iteration)",
                       "load_column": "from zero" if args.no_warm_start else
                                      "warm start from the previous Newton iteration's solution",
                       "material": "NeoHooke E=1000 nu=0.3", "l2": "256 MB buffer written before each timed path"}}
@@ -1038,7 +1036,9 @@ def run_path_following(args):
                     "cg_iterations": info.totalLinearIterations,
                     "newton_per_step": [si.iterations for si in info.solverInfos],
                     "final_lambda": req.parameter(), "psi": pf.subsidiary_args()["psi"], **pf.stats(),
-                    "spmv_kernel": ls.kernel_info()[:2]}
+                    "spmv_kernel": ls.kernel_info()[:2],
+                    "bordered_solves": dict(zip(("one_launch_for_both_columns", "one_column_after_the_other"),
+                                                ls.multi_rhs_info()))}
         finals[key] = req.globalSolution()
         del pf, nr, ls, req, asm, fes
     out["value"] = out["mixed"]["s"]

@@ -260,6 +260,7 @@ SIGNATURES = {
     "ikr_load_control_run": ([_vp, _vp, C.POINTER(_ControlInfo), C.POINTER(_NRInfo), _I], C.c_int),
     "ikr_load_control_set_predictor": ([_vp, _I, _vp, _dp, _I], C.c_int),
     "ikr_linear_solver_set_multi_rhs": ([_vp, _I], C.c_int),
+    "ikr_linear_solver_multi_rhs_info": ([_vp, _i64p, _i64p], C.c_int),
     "ikr_linear_solver_set_coarse_space": ([_vp, _I], C.c_int),
     "ikr_linear_solver_coarse_info": ([_vp, _ip], C.c_int),
     "ikr_linear_solver_set_coarse_refresh": ([_vp, _I], C.c_int),
@@ -1091,9 +1092,16 @@ class LinearSolver:
         _err(lib().ikr_linear_solver_set_kernel(self.h, int(spmv_kind), float(l2_keep_fraction)))
 
     def set_multi_rhs(self, on=True):
-        """Two right-hand sides with one tangent (path following): one persistent launch streaming the matrix once
-        per iteration for both (default), or one solve after the other."""
+        """Two right-hand sides with one tangent (path following): with a two-barrier persistent CG kind on an FP32
+        tangent one launch streaming the matrix once per iteration for both (default), or one solve after the other.  The
+        other kinds, the one-reduction CG among them, solve one after the other."""
         _err(lib().ikr_linear_solver_set_multi_rhs(self.h, int(bool(on))))
+
+    def multi_rhs_info(self):
+        """(solves with two right-hand sides since creation in one launch, one after the other)."""
+        a, b = C.c_int64(), C.c_int64()
+        _err(lib().ikr_linear_solver_multi_rhs_info(self.h, C.byref(a), C.byref(b)))
+        return a.value, b.value
 
     def set_fp64_outer(self, restart=20, inner_rtol=1e-2, inner_max_iter=2000, outer_max_iter=2000):
         """FP64 outer solve of an FP32 tangent (restart 0 switches it off): flexible GMRES(restart) on the FP64

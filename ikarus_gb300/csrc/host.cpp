@@ -1167,6 +1167,12 @@ int ikr_linear_solver_set_multi_rhs(ikr_ls ls, int32_t on) {
     ls->multi_rhs = on != 0;
   });
 }
+int ikr_linear_solver_multi_rhs_info(ikr_ls ls, int64_t* one_launch, int64_t* one_after_the_other) {
+  return guarded([&] {
+    need(ls && one_launch && one_after_the_other, IKR_ERR_ARG, "null argument");
+    *one_launch = ls->two_rhs[0], *one_after_the_other = ls->two_rhs[1];
+  });
+}
 int ikr_linear_solver_set_coarse_space(ikr_ls ls, int32_t n_slabs) {
   return guarded([&] {
     need(ls, IKR_ERR_ARG, "null argument");

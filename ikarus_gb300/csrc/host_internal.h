@@ -538,6 +538,7 @@ struct ikr_ls_s {
   // second right-hand side of solve2 (its own CG vectors and scalars; matrix, preconditioner, grid and L2
   // policy are w's) and the partials of the two-RHS persistent kernel (4 and 8 per CTA)
   bool multi_rhs = true;
+  int64_t two_rhs[2] = {0, 0};  // solves with two right-hand sides in one launch, one after the other
   ikr::PcgWork w2;
   // Coarse correction of the CG (coarse.cu), off by default: coarse_req > 0 slab aggregates of equal node
   // count along the mesh's longest extent, six rigid-body modes each; rebuilt (A_c and its inverse) at every
@@ -1230,9 +1231,12 @@ struct ikr_ls_s {
     pb2.alloc(8 * (size_t)w.grid);
   }
 
-  // x0 = K^{-1} b0 and x1 = K^{-1} b1 with the same tangent.  With a persistent CG kind both run in one
+  // x0 = K^{-1} b0 and x1 = K^{-1} b1 with the same tangent.  With a two-barrier persistent CG kind both run in one
   // cooperative launch that streams the matrix once per iteration for the two; otherwise (or with refinement
-  // sweeps, or when disabled) one solve after the other.  Returns the CG iterations of both right-hand sides.
+  // sweeps, or when disabled) one solve after the other.  Two solves of the one-reduction kind are faster than the common
+  // launch at every size: arc-length steps, microseconds per CG iteration of a column, one after the other against the best
+  // common launch: 425 rows 7.2 / 21.0, 18 785 10.8 / 23.6, 60 625 15.5 / 29.1; 140 481 rows, four steps, 2.09 / 2.44 s.
+  // Returns the CG iterations of both right-hand sides.
   int64_t solve2(ikr_asm a, const double* b0, const double* b1, double* x0, double* x1, double rt, int maxit,
                  int refinements, double rt1 = -1.0) {
     if (rt1 < 0.0) rt1 = rt;
@@ -1248,6 +1252,7 @@ struct ikr_ls_s {
       w2.minv = w.minv, w2.keep_g = w.keep_g, w2.spmv_kind = w.spmv_kind;
       two = ikr::pcg_persistent2_eligible(A, w, w2, w.spmv_kind - first_persistent_kind());
     }
+    ++two_rhs[two ? 0 : 1];
     if (!two) {
       const int64_t i0 = solve(a, b0, x0, rt, maxit, refinements);
       const int64_t i1 = solve(a, b1, x1, rt1, maxit, refinements);

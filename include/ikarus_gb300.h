@@ -295,10 +295,13 @@ int ikr_assembler_tangent_kernel(ikr_asm a, int32_t* path);
 /* no reference counterpart, for tests: gathered tangents (FP64 and EAS ones, kernel 3 of the FP32 ones) hold the blocks or
  * matrices of at most this many elements at a time; 0 (default): 4 GB of them.  The tangent does not depend on it. */
 int ikr_assembler_set_gather_part(ikr_asm a, int64_t n_elems);
-/* no reference counterpart: solves with two right-hand sides and one tangent (path following's bordered
- * system) run both CGs in one persistent launch that streams the matrix once per iteration (on = 1, default)
- * or one after the other (0) */
+/* no reference counterpart: solves with two right-hand sides and one tangent (path following's bordered system).  With
+ * one of the two-barrier persistent CG kinds on an FP32 tangent both CGs run in one launch that streams the matrix once
+ * per iteration (on = 1, default) or one after the other (0); the other kinds, the one-reduction CG among them, always solve
+ * one after the other (its two solves take about half the time of the common launch).  multi_rhs_info: such solves since
+ * creation in one launch and one after the other. */
 int ikr_linear_solver_set_multi_rhs(ikr_ls ls, int32_t on);
+int ikr_linear_solver_multi_rhs_info(ikr_ls ls, int64_t* one_launch, int64_t* one_after_the_other);
 int ikr_linear_solver_kernel_info(ikr_ls ls, int32_t* spmv_kind, double* l2_keep_fraction, double* spmv_us);
 /* no reference counterpart: coarse correction of IKR_SOLVER_GPU_PCG_BLOCK_JACOBI (off by default, n_slabs = 0).
  * n_slabs in [1, 128] adds P A_c^-1 P^T to the block-Jacobi preconditioner, an additive two-level method: the
