@@ -812,14 +812,15 @@ __global__ void __launch_bounds__(WARPS * 32, 1) pcg_halo_kernel(const __grid_co
       for (int c = 0; c < NC; ++c) H.x[4 * (int64_t)(row0 + row_of(j)) + comp + c] = xr[j][c];
     }
   if (tid == 0 && (cta == 0 || failed)) {
-    // a CTA that gave up says so itself: CTA 0 may have finished before it
+    // a CTA that gave up says so itself, and CTA 0 may have finished before or after it: the largest status stays (as bits,
+    // statuses are not negative)
     if (cta == 0) {
       H.scal[kIters] = (double)it;
       H.scal[kRR] = rrs;
       H.scal[kRz] = rz;
       H.scal[kBeta] = beta;
     }
-    H.scal[kDone] = failed ? kDoneDeviceTimeout : (double)done;
+    atomicMax(reinterpret_cast<long long*>(H.scal + kDone), __double_as_longlong(failed ? kDoneDeviceTimeout : (double)done));
   }
 }
 
