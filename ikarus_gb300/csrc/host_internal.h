@@ -325,6 +325,10 @@ struct ikr_req_s {
 };
 
 struct ikr_asm_s {
+  const uint64_t id = [] {  // of every assembler of this process: an address may come back
+    static std::atomic<uint64_t> made{0};
+    return ++made;
+  }();
   ikr_fes fes = nullptr;
   int n = 0, nred = 0;
   bool fp32 = false;
@@ -495,6 +499,8 @@ struct ikr_ls_s {
   double rtol = 1e-10;
   int max_iter = 100000;
   ikr_asm asm_ = nullptr;
+  uint64_t asm_id = 0;
+  bool holds(ikr_asm a) const { return factorized && asm_ == a && asm_id == a->id; }
   bool fp32 = false;
   ikr::PcgWork w;
   DBuf<double> dx, dp, dq, dmv, pa, pb, scal;
@@ -599,9 +605,10 @@ struct ikr_ls_s {
 
   void setup(ikr_asm a) {
     a->dual64 = outer_m > 0 && a->fp32;  // the FP64 outer solve needs the FP64 twin of every later assembly
-    if (asm_ == a && w.n_rows == a->fes->nn && fp32 == a->fp32 && w.grid) return;
+    if (asm_ == a && asm_id == a->id && w.n_rows == a->fes->nn && fp32 == a->fp32 && w.grid) return;
     drop_graphs();
-    asm_ = a;
+    asm_ = a, asm_id = a->id;
+    co.built_for = nullptr;
     fp32 = a->fp32;
     const int nr = a->fes->nn;
     const size_t n = 4 * (size_t)nr;  // CG vectors are node-padded (x, y, z, 0)
@@ -1163,7 +1170,7 @@ struct ikr_ls_s {
 
   // x = K^{-1} b on the device (FP64 in / out); returns CG iterations
   int solve_device(ikr_asm a, const double* b, double* x, double rt, int maxit) {
-    if (!factorized || asm_ != a) fail(IKR_ERR_INVALID_STATE, "linear solver not factorized for this assembler");
+    if (!holds(a)) fail(IKR_ERR_INVALID_STATE, "linear solver not factorized for this assembler");
     if (persistent()) return solve_persistent(a, b, x, rt, maxit);
     if (coarse_fused()) return solve_coarse_fused(a, b, x, rt, maxit);
     cudaStream_t s = a->fes->stream;
@@ -1241,7 +1248,7 @@ struct ikr_ls_s {
                  int refinements, double rt1 = -1.0) {
     if (rt1 < 0.0) rt1 = rt;
     if (direct) rt = std::min(rt, rtol), rt1 = std::min(rt1, rtol);
-    if (!factorized || asm_ != a) fail(IKR_ERR_INVALID_STATE, "linear solver not factorized for this assembler");
+    if (!holds(a)) fail(IKR_ERR_INVALID_STATE, "linear solver not factorized for this assembler");
     const ikr::Bsr A = a->bsr();
     // FP64 CG iterations are bound by GB300's FP64 pipe, not by the matrix stream: two right-hand sides cost
     // twice the time in one launch as well, so only the FP32 tangent runs them together (and only without the

@@ -23,7 +23,7 @@ bool step_graph_eligible(ikr_nr nr, ikr_req r) {
   const ikr_nr_settings& st = nr->st;
   if (!st.step_graphs || (nr->step_graph && nr->step_graph->unsupported)) return false;
   return r->fes == f && f->na == 0 && f->n_inst == 0 && !a->has_idbc && !a->dual64 && st.refinements <= 0 &&
-         st.max_backtracks <= 0 && ls->tag != IKR_SOLVER_GPU_PCG_BATCHED && ls->factorized && ls->asm_ == a &&
+         st.max_backtracks <= 0 && ls->tag != IKR_SOLVER_GPU_PCG_BATCHED && ls->holds(a) &&
          ls->tuned_for == a && ls->persistent() && !ls->w.coarse && ls->outer_m == 0 && !ls->direct && !ls->profile &&
          f->epb_r > 0 && (a->fp32 ? f->epb_k32 : f->epb_k64) > 0 && (!a->fp32 || a->tan_path > 0) && a->nb > 0 &&
          !f->trac_dirty;
