@@ -763,13 +763,14 @@ void launch_residual_gp(const ElemArgs& a, const int32_t* list, int n_list, int 
 constexpr int kTanPoint = 49;                    // doubles of a point: 8 nodes x (dN, g), padded against bank conflicts
 constexpr int kTanElem = 8 * kTanPoint + 3 * 8;  // and the weights of the eight points
 template <bool FULL>
-__global__ void __launch_bounds__(32) tangent64_kernel(ElemArgs a, int n_list, int e_base) {
+__global__ void __launch_bounds__(32) tangent64_kernel(ElemArgs a, const int32_t* __restrict__ list, int n_list,
+                                                       int e_base) {
   __shared__ __align__(16) double sm[4 * kTanElem];
   const int lane = threadIdx.x, sub = lane & 7, es = lane >> 3, src = lane & ~7;
   const int li = blockIdx.x * 4 + es;
   const bool active = li < n_list;
   const int lic = active ? li : n_list - 1;
-  const int e = e_base + lic;
+  const int e = list ? list[lic] : e_base + lic;
   const int ne = a.n_elems;
   const int node = a.conn[sub * ne + e];
   double dX[3], dU[3];
@@ -902,8 +903,8 @@ __global__ void __launch_bounds__(32) tangent64_kernel(ElemArgs a, int n_list, i
 // and 0.06 ms for the gather, 81 % of it FP64 instructions by count; 256 elements 1.24 ms (eight dependent launches of
 // 155 us) -> 50 and 9 us.
 template <bool FULL>
-void launch_tangent64(const ElemArgs& a, int n_list, int e_base, cudaStream_t s) {
-  tangent64_kernel<FULL><<<(n_list + 3) / 4, 32, 0, s>>>(a, n_list, e_base);
+void launch_tangent64(const ElemArgs& a, const int32_t* list, int n_list, int e_base, cudaStream_t s) {
+  tangent64_kernel<FULL><<<(n_list + 3) / 4, 32, 0, s>>>(a, list, n_list, e_base);
 }
 
 // calculateAt<PK2Stress / kirchhoffStress / cauchyStress> (nonlinearelastic.hh:237-271) of elements
@@ -1190,7 +1191,7 @@ void launch_disp_element(const ElemArgs& a, int mode, bool fp32_tangent, const i
       break;
     case kWantK: launch_disp_t<float, kWantK>(a, list, n_list, e_base, s); break;  // coloured, FP32
     case kWantK | kElemOut:
-      if (a.material == 0) launch_tangent64<true>(a, n_list, e_base, s);
+      if (a.material == 0) launch_tangent64<true>(a, list, n_list, e_base, s);
       else if (a.material == 1) launch_disp_epb<double, kWantK | kElemOut, 32, 1>(a, list, n_list, e_base, s);
       else if (a.material == 2) launch_disp_epb<double, kWantK | kElemOut, 32, 2>(a, list, n_list, e_base, s);
       else launch_disp_epb<double, kWantK | kElemOut, 32, 3>(a, list, n_list, e_base, s);
@@ -1198,7 +1199,7 @@ void launch_disp_element(const ElemArgs& a, int mode, bool fp32_tangent, const i
     case kWantEnergy | kElemOut: launch_disp_t<double, kWantEnergy | kElemOut>(a, list, n_list, e_base, s); break;
     case kWantK | kElemBlocks:
       if (fp32_tangent) launch_disp_t<float, kWantK | kElemBlocks>(a, list, n_list, e_base, s);
-      else launch_tangent64<false>(a, n_list, e_base, s);  // NeoHooke, all elements
+      else launch_tangent64<false>(a, list, n_list, e_base, s);  // NeoHooke
       break;
     default: break;
   }
