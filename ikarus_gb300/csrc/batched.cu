@@ -19,7 +19,7 @@
 // state in the work arrays); batched_pcg_smem_kernel with four, eight or sixteen threads per row and the CTA's
 // matrix blocks in shared memory; and, in FP32, batched_pcg_cluster_kernel with one instance per thread-block
 // cluster and its vectors in distributed shared memory.  A planner left its choice runs the GROUPS form of cg_halo.cu
-// instead where that fits (an instance set of at most one CTA per SM): 128 instances of 60 000 rows in all, FP32, took
+// instead where that fits (at most twice as many instances as SMs, in one launch or two): 128 instances of 60 000 rows in all, FP32, took
 // 16 to 20 us per iteration here and 10 there, less as instances finish.  Every wait on a global barrier is bounded; a wait that gives
 // up ends the instance with flag -1.
 #include <map>

@@ -23,13 +23,18 @@
 //     total is as good as one of doubles; it does not depend on an order.
 // Measured, microseconds per iteration, the best of the two-barrier forms -> this kernel:
 //   rows        44            425           2 673         18 785        35 721        140 481
-//   FP32   10.3 ->  3.6  13.6 ->  4.1  13.9 ->  4.4  14.2 ->  6.0  14.5 ->  7.9  29.7 -> 23.3
-//   FP64   16.3 ->  4.7  36.1 ->  5.5  38.9 ->  7.0  39.8 -> 15.0  39.8 -> 24.3   128 ->   77
+//   FP32    6.6 ->  3.7  13.6 ->  4.1  13.5 ->  4.5  14.1 ->  6.3  14.3 ->  8.1  29.1 -> 23.6
+//   FP64   17.0 ->  4.9  36.4 ->  5.7  38.9 ->  6.8  39.7 -> 15.0  39.5 -> 24.4   127 ->   78
+// Node numberings cost it less than the two-barrier forms (nodes shuffled throughout, 18 785 rows FP32 22.1 -> 7.2, FP64
+// 41.2 -> 18.7; 35 721 rows 23.1 -> 14.5 and 41.2 -> 36.3, the closest of 50 combinations of size, numbering and
+// precision; 80 625 rows shuffled within 512 nodes 27.1 -> 17.0 and 82 -> 53.5).
 // The small sizes are bound by two trips through L2 (p to the neighbours, the sums to everyone) and the chains between
 // them, FP64 from 18 785 rows on by the FP64 pipe (nine multiply-adds per block: 8, 15 and 54 us of the last three), FP32
-// at 140 481 rows by the 152 MB of blocks streamed through L2.
-// GROUPS: the same for many independent instances, a group of CTAs each (plan_halo_launch in batched_host.cpp).  A load
-// step of 128 instances in mixed precision 227 -> 117 ms, of 100 in FP64 819 -> 383 ms against the kernels of batched.cu.
+// at 140 481 rows by the 118 MB of blocks streamed through L2, 72 MB of them from DRAM (45 % of the copy bandwidth); the
+// other fifth of the matrix stays in shared memory.
+// GROUPS: the same for many independent instances, a group of CTAs each (plan_halo in batched_host.cpp).  A load step
+// of 128 instances in mixed precision (mean of four) 241 -> 131 ms, of 300 472 -> 291 ms, of 100 in FP64 (two) 789 -> 269 ms
+// against the kernels of batched.cu.
 // The launch is cooperative (all CTAs co-resident) and every wait is bounded: one that gives up ends the CTA with
 // scal[kDone] = 6 after its copies in flight have been drained, and with it the waits of the others.
 #include <algorithm>
@@ -695,8 +700,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1) pcg_halo_kernel(const __grid_co
       }
       if (__any_sync(0xffffffffu, pend != 0) && lane == 0) s_fail = 1;
       __syncwarp();
-      // five normalised numbers below 2^61 per lane, a sixteenth of each: below 2^59.4 and, of 160, below 2^62 after
-      // the three bits that warp_sum's bound asks for
+      // five normalised numbers below 2^61 per lane, a sixty-fourth of each: below 2^57.4, inside warp_sum's bound
       int X = kZeroExp;
 #pragma unroll
       for (int j = 0; j < kMaxCtas / 32; ++j) X = max(X, t[j].x);

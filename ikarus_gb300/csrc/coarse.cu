@@ -19,7 +19,7 @@
 // instructions per block, the translations being additions), then P_I^T W, a CTA its 256 rows, and a second kernel the
 // CTAs of an aggregate in order.  The host symmetrises A_c and inverts it (ikr_ls_s in host_internal.h).  All sums are
 // fixed-order: results are bit-identical run to run.  Measured at 140 481 rows, three distances: 18 probe products
-// K V_m (164 us each, the matrix read 18 times) and their restrictions took 3.3 ms, this pass 0.83 ms.
+// K V_m (164 us each, the matrix read 18 times) and their restrictions took 3.3 ms, this pass 0.47 ms.
 #include "cg_common.cuh"
 
 namespace ikr {

@@ -807,8 +807,8 @@ struct ikr_ls_s {
       const int32_t bits = agg[i] | (mask << 24);
       std::memcpy(&y4[4 * i + 3], &bits, sizeof(bits));
     }
-    // reach: the largest aggregate distance of two coupled nodes; colours of a distance-2 colouring of the
-    // aggregate chain (any 2 reach + 1 consecutive aggregates differ)
+    // reach: the largest aggregate distance of two coupled nodes.  (The colours of a distance-2 colouring of the chain, any
+    // 2 reach + 1 consecutive aggregates, are only reported.)
     int reach = 0;
     for (int i = 0; i < nn; ++i)
       for (int k = a->row_ptr_h[i]; k < a->row_ptr_h[i + 1]; ++k) reach = std::max(reach, std::abs(agg[i] - agg[a->col_h[k]]));
@@ -1043,8 +1043,8 @@ struct ikr_ls_s {
     if (spmv_req < 0) {
       // the kinds are compared with a mid L2 keep share (the share changes their ranking), kind 0 has none
       constexpr double kProbeKeep = 0.45;
-      // The one-reduction kernel wherever a split fits: it was the fastest persistent form at every size timed (table
-      // in cg_halo.cu), so only its variants are compared
+      // The one-reduction kernel wherever a split fits: it was the fastest kind at every size and node numbering timed
+      // (figures in cg_halo.cu), so only its variants are compared
       bool halo = false;
       for (int v = 0; v < ikr::kHaloVariants && coarse_req == 0; ++v) {
         if (!ikr::pcg_halo_eligible(w, v)) continue;
