@@ -11,7 +11,9 @@
 // factorising D keeps the other seven.  The loops over modes, columns and blocks are rolled: unrolled, the kernels had 120 to
 // 280 KB of instructions, each run once, and now have 70 to 120.  Measured with assembly, residual and tangent, eight
 // lanes per element and one launch per colour -> unrolled -> this: 10 elements (H9) 660 -> 60 -> 46 us and 1 030 -> 80 -> 67 us,
-// 8 192 elements (E9) 2.34 -> 1.01 -> 0.75 ms and 3.86 -> 1.63 -> 1.35 ms.
+// 8 192 elements (E9) 2.34 -> 1.01 -> 0.75 ms and 3.86 -> 1.63 -> 1.35 ms.  E21, whose tangent takes 110 KB of shared memory,
+// two blocks per SM, first and last form: 256 elements 6.53 -> 0.12 and 8.32 -> 0.14 ms, 16 384 elements 6.96 -> 4.74 and
+// 8.88 -> 6.12 ms.
 // The lanes of a point share F, S and the Voigt tangent C (each lane computes a few of its 36 entries into shared
 // memory), and each lane computes the enhanced-strain columns E_alpha(:,k) and C E_alpha(:,k) for k = I, I+8, ...
 // The points' shares of f, K, L, D and R~ are summed in a fixed order through shared memory.  D (n_alpha x n_alpha) is

@@ -79,18 +79,18 @@ void need(bool c, int code, const char* msg) {
 // EAS condensation cache key: valid while the same requirement, solution and alpha are in place
 uint64_t cache_key(ikr_req r, ikr_fes f) { return (r->id * 0x9E3779B97F4A7C15ull) ^ (r->version << 20) ^ f->alpha_version; }
 
-// Elements per block of the displacement element kernel: each of 16, 32 and 64 is timed once on a complete
+// Elements per block of the displacement element kernel: each of `sizes` is timed once on a complete
 // pass of the given kind and the fastest is kept for the element set (the choice does not change any
 // result: the summation order does not depend on it).  `pass` runs one pass with args.epb.
 template <typename Pass>
-static int choose_epb(ikr_fes f, Pass pass) {
+static int choose_epb(ikr_fes f, std::initializer_list<int> sizes, Pass pass) {
   if (f->na > 0) return 32;  // the EAS kernel has its own launch shape
   cudaEvent_t e0, e1;
   CK(cudaEventCreate(&e0));
   CK(cudaEventCreate(&e1));
   int best = 32;
   float best_ms = 1e30f;
-  for (int epb : {16, 32, 64}) {
+  for (int epb : sizes) {
     pass(epb);  // warm
     CK(cudaEventRecord(e0, f->stream));
     pass(epb);
@@ -121,7 +121,8 @@ void assemble_vector(ikr_asm a, ikr_req r, int dbc, bool sync) {
   args.elem_vec = f->fel.p;
   constexpr int kMode = ikr::kWantR | ikr::kElemOut;
   if (!f->epb_r) {
-    f->epb_r = choose_epb(f, [&](int epb) {
+    // (the launch has one shape up to 4 096 elements, two above)
+    f->epb_r = f->ne <= 4096 ? 32 : choose_epb(f, {16, 32}, [&](int epb) {
       ikr::ElemArgs t = args;
       t.epb = epb;
       f->launch_elements(t, kMode, false, nullptr, f->ne, 0);
@@ -174,7 +175,7 @@ static void assemble_matrix32(ikr_asm a, ikr::ElemArgs& args, const uint8_t* nf)
   ikr_fes f = a->fes;
   int& epb_k = f->epb_k32;
   if (!epb_k) {
-    epb_k = choose_epb(f, [&](int epb) {
+    epb_k = choose_epb(f, {16, 32, 64}, [&](int epb) {
       ikr::launch_bsr_reset(a->values(), true, a->npad, a->diag.p, nf, f->nn, f->stream);
       ikr::ElemArgs t = args;
       t.epb = epb;
